@@ -271,7 +271,7 @@ cudaError_t launch_gemm_bf16_tc(const uint16_t *x, int M, int K, const uint16_t 
   if (M <= 0 || N <= 0 || N % 8 != 0 || K <= 0 || K % 8 != 0)
     return cudaErrorInvalidValue;
   if (spin_limit == 0)
-    spin_limit = 1u << 26; // about a second
+    spin_limit = tc::kSpinLimit;
   CUtensorMap map_x, map_w;
   if (!bf16_map(&map_x, x, M, K) || !bf16_map(&map_w, w, N, K))
     return cudaErrorNotSupported;

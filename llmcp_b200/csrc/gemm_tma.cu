@@ -14,21 +14,27 @@
 //         2^19, both exact in f32, so the tensor core hands back float(dot) itself, bit for bit what
 //         the conversion would give, and the epilogue is multiply + fma.  The price is operand planes
 //         of twice the size in HBM and on the way from L2.
-// Either form optionally with two-lane f32x2 multiplies and fmas (same roundings, half the
-// instructions).  Measured on 1024 x 9216 x 2560: int8 199 us, int8 packed 177 us, f16 191 us,
-// f16 packed 181 us (the cp.async-fed kernel of gemm_tc.cu: 222 us); what remains is the epilogue
-// warps' instruction issue and the hand-off per block, not the tensor pipe (under 10 % busy).
+// Both forms multiply and add with two-lane f32x2 instructions (same roundings, half the instructions).
 //
-// One CTA per 128 x 128 output tile, 576 threads:
+// What bounds it: the epilogue warps, 3 (int8) or 2 (f16) instructions' worth of lanes per (row, column, block), and
+// the hand-off between them and the tensor core; the tensor pipe is under 10 % busy.  Loads from tensor memory,
+// conversion, scales and fmas alone take 430 cycles per 128 x 128 x 32 block on an SM (346 without the conversion);
+// handing over every block by itself made it 1000.  Two blocks per hand-off, descriptors advanced by an add, one
+// elected lane per role (so that the compiler knows it is one) and a persistent grid (a tile's output is stored while
+// the next tile's blocks are already multiplied) bring it to 800: 1024 x 9216 x 2560 170 -> 130 us, 1024 x 2560 x 4096
+// 87 -> 84, 1024 x 32 x 2560 42 -> 22.  Fragment-shaped tensor-memory loads (16x256b: fewer scale registers) read
+// tensor memory at a quarter of the rate and measured 160 us.
+//
+// One CTA per SM takes 128 x TN output tiles in turn, 576 threads:
 //   warp  0     one lane issues the TMA loads (cp.async.bulk.tensor, 128-byte swizzle, no
-//               multicast): per stage a box of 128 rows x 128 bytes of K of each operand (four
+//               multicast): per stage a box of 128 (TN) rows x 128 bytes of K of each operand (four
 //               int8 or two f16 quantisation blocks) and those blocks' f32 scales of the tile's rows
-//               and columns (scale planes are block-major, [K/32][rows], so a box is 128 consecutive
+//               and columns (scale planes are block-major, [K/32][rows], so a box is consecutive
 //               floats per block);
-//   warp  1     one lane issues the MMAs into tensor-memory buffer kb % 4 (f16: two K = 16
-//               instructions per block, the first overwrites, the second accumulates);
-//   warps 2-17  epilogue: tcgen05.ld the buffer (thread = row, 32 columns), hand the buffer back,
-//               then the arithmetic with the scales read from shared memory.
+//   warp  1     one lane issues the MMAs, two blocks into a tensor-memory slot (f16: two K = 16
+//               instructions per block, the first overwrites, the second accumulates), and commits the slot;
+//   warps 2-17  epilogue: tcgen05.ld a block (thread = row, TN / 4 columns), hand the slot back after its last
+//               block's load, then the arithmetic with the scales read from shared memory.
 // Hand-offs are mbarriers; every wait is bounded (spin_limit polls) and a timed-out wait raises an
 // abort flag that all roles observe, so a protocol error ends the kernel with an error code instead
 // of hanging it; the loader then waits (bounded) for the copies it has in flight.  Tensor memory
@@ -49,33 +55,31 @@ namespace {
 using namespace tc;
 
 constexpr int kTileM = 128;
-// Output tiles are 128 rows by TN columns, TN = 128 (four tensor-memory buffers) or 160 (three): the
-// wider tile exists for matrices whose 128-wide tiles would leave a nearly empty last wave (N = 2560 at
-// 1024 rows: 160 tiles on 148 SMs, against 128 tiles of 160 columns in one wave).
-template <int TN> struct Tile {
-  static_assert(TN == 128 || TN == 160, "tile widths with a tensor-memory plan");
-  static constexpr int kBuffers = TN == 128 ? 4 : 3;  // TN columns of 32-bit accumulators each, 512 in all
-  static constexpr int kStages = TN == 128 ? 6 : 5;
-  static constexpr int kWarpColumns = TN / 4;         // columns per epilogue warp: 32, or 32 + 8
-  static constexpr int kOperandBytesB = TN * 128;
-};
-constexpr int kMaxBuffers = 4, kMaxStages = 6;
 constexpr int kEpilogueWarp0 = 2;
 constexpr int kEpilogueWarps = 16;
 constexpr int kThreads = 32 * (kEpilogueWarp0 + kEpilogueWarps);
-constexpr int kOperandBytes = kTileM * 128;  // 16 KB per operand per stage: rows of 128 bytes of K
+constexpr int kOperandBytes = kTileM * 128; // 16 KB of activations per stage: rows of 128 bytes of K
+constexpr int kMaxSlots = 4, kMaxStages = 6;
 constexpr int kBarrierBytes = 256;
 
-// F16: operands are f16 values (64 per 128-byte row = 2 quantisation blocks per stage);
-// otherwise int8 (128 per row = 4 blocks per stage).
-template <bool F16, int TN = 128> struct Form {
+// Tiles of 128 rows by TN columns.  F16: operands are f16 values (64 per 128-byte row = 2 quantisation blocks per
+// stage); otherwise int8 (128 per row = 4 blocks per stage).  Tensor memory holds kSlots slots of kSlotBlocks blocks'
+// dots each; a slot is handed over as a whole.
+template <bool F16, int TN> struct Form {
+  static_assert(TN == 64 || TN == 96 || TN == 128, "tile widths with a tensor-memory plan");
+  static constexpr int kSlotBlocks = 2;
+  static constexpr int kSlots = 512 / (kSlotBlocks * TN);
+  static constexpr int kWarpColumns = TN / 4;                       // columns per epilogue warp: 16, 24 or 32
+  static constexpr int kStages = TN >= 128 ? 5 : 6;
   static constexpr int kStageBlocks = F16 ? 2 : 4;
   static constexpr int kStageK = kStageBlocks * 32;                 // elements of K per stage
+  static constexpr int kOperandBytesB = TN * 128;
   static constexpr int kScaleBytesA = kStageBlocks * kTileM * 4;    // the rows' scales of a stage
   static constexpr int kScaleBytesB = kStageBlocks * TN * 4;        // the columns' scales
-  static constexpr int kScaleBytes = (kScaleBytesA + kScaleBytesB + 1023) / 1024 * 1024;
-  static constexpr int kStageBytes = kOperandBytes + Tile<TN>::kOperandBytesB + kScaleBytes; // multiples of 1024
-  static constexpr size_t kSmemBytes = 1024 + Tile<TN>::kStages * kStageBytes + kBarrierBytes;
+  static constexpr int kCopied = kOperandBytes + kOperandBytesB + kScaleBytesA + kScaleBytesB;
+  static constexpr int kStageBytes = (kCopied + 1023) / 1024 * 1024;
+  static constexpr size_t kSmemBytes = 1024 + kStages * kStageBytes + kBarrierBytes;
+  static_assert(kSmemBytes <= 227 * 1024 && kSlots >= 2 && kSlots <= kMaxSlots, "plan of a CTA");
 };
 
 // kind::f16: f16 x f16 -> f32, both operands K-major, M = 128, N = TN, K = 16 per instruction.
@@ -101,57 +105,78 @@ __device__ __forceinline__ void mma_i8(uint32_t tmem, uint64_t a, uint64_t b, ui
                : "memory");
 }
 
-// Two f32 lanes per instruction (each lane rounds as the scalar instruction does).
-__device__ __forceinline__ void mul2(float &d0, float &d1, float a0, float a1, float b0, float b1) {
-  asm("{ .reg .b64 a, b, d; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; mul.rn.f32x2 d, a, b; mov.b64 {%0, %1}, d; }"
-      : "=f"(d0), "=f"(d1)
-      : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
+// COLUMNS consecutive 32-bit columns of this thread's lane.
+template <int COLUMNS> __device__ __forceinline__ void tmem_load_columns(uint32_t taddr, uint32_t (&r)[COLUMNS]) {
+  if constexpr (COLUMNS >= 32)
+    tmem_issue32(taddr, *reinterpret_cast<uint32_t(*)[32]>(r));
+  else
+    tmem_issue16(taddr, *reinterpret_cast<uint32_t(*)[16]>(r));
+  if constexpr (COLUMNS % 16 == 8)
+    tmem_issue8(taddr + COLUMNS - 8, *reinterpret_cast<uint32_t(*)[8]>(r + COLUMNS - 8));
+  tmem_wait_loads_into(r);
 }
-__device__ __forceinline__ void fma2(float &c0, float &c1, float a0, float a1, float b0, float b1) {
-  asm("{ .reg .b64 a, b, c; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; mov.b64 c, {%0, %1}; fma.rn.f32x2 c, a, b, c; mov.b64 {%0, %1}, c; }"
+
+// c += v * (a * w), two columns at a time; every lane of the pair rounds as the scalar instructions do.
+__device__ __forceinline__ void fold2(float &c0, float &c1, float v0, float v1, float a, float w0, float w1) {
+  asm("{ .reg .b64 s, w, v, c; mov.b64 s, {%2, %2}; mov.b64 w, {%3, %4}; mul.rn.f32x2 s, s, w; mov.b64 v, {%5, %6};\n"
+      "mov.b64 c, {%0, %1}; fma.rn.f32x2 c, v, s, c; mov.b64 {%0, %1}, c; }"
       : "+f"(c0), "+f"(c1)
-      : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
+      : "f"(a), "f"(w0), "f"(w1), "f"(v0), "f"(v1));
 }
+
+// mbar_wait by a whole warp: all lanes get the same answer.
+__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag, uint32_t limit) {
+  return __all_sync(0xffffffffu, mbar_poll(smem_u32(bar), parity)) ||
+         __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, limit));
+}
+
+// A position in a ring of `size` barriers and the parity of its current phase.
+struct Ring {
+  int at = 0;
+  uint32_t parity = 0;
+  __device__ __forceinline__ void next(int size) {
+    if (++at == size)
+      at = 0, parity ^= 1;
+  }
+};
 
 struct Barriers {
   uint64_t full[kMaxStages];     // stage landed in shared memory (one arrival + the copies' bytes)
   uint64_t empty[kMaxStages];    // stage no longer needed: MMA done (1) + every epilogue warp (scales read)
-  uint64_t tfull[kMaxBuffers];   // a block's dot products are in the tensor-memory buffer
-  uint64_t tempty[kMaxBuffers];  // the buffer has been read by all epilogue warps
+  uint64_t tfull[kMaxSlots];     // the slot's dot products are in tensor memory
+  uint64_t tempty[kMaxSlots];    // the slot has been read by all epilogue warps
   uint64_t done;                 // the last commit of the MMA lane has arrived (see the end of its loop)
   uint32_t tmem_base;
   int abort_flag;
 };
+static_assert(sizeof(Barriers) <= kBarrierBytes, "barriers");
 
 // fault (test hook): 1 = the loader announces the first stage's bytes but never issues its copies,
 // so the barrier of that stage cannot complete and every wait behind it has to run out.
-// PACKED: the epilogue's multiplies and fmas as two-lane f32x2 instructions (same roundings).
-template <bool F16, bool PACKED, bool DOTS, int TN>
+template <bool F16, bool DOTS, int TN>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_q8_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const __grid_constant__ CUtensorMap map_as, const __grid_constant__ CUtensorMap map_bs, int M, int K,
-                    int N, void *__restrict__ y, int y_dtype, int activation, int32_t *__restrict__ dots_out,
-                    int *__restrict__ error_out, uint32_t spin_limit, int fault) {
+                    int N, int tiles, int m_tiles, void *__restrict__ y, int y_dtype, int activation,
+                    int32_t *__restrict__ dots_out, int *__restrict__ error_out, uint32_t spin_limit, int fault) {
   using F = Form<F16, TN>;
-  constexpr int kStageBlocks = F::kStageBlocks, kStageK = F::kStageK, kStageBytes = F::kStageBytes;
-  constexpr int kTileN = TN, kTmemBuffers = Tile<TN>::kBuffers, kStages = Tile<TN>::kStages, kWarpColumns = Tile<TN>::kWarpColumns;
-  constexpr int kOperandBytesB = Tile<TN>::kOperandBytesB;
+  constexpr int kStageBlocks = F::kStageBlocks, kStages = F::kStages, kSlots = F::kSlots, kSlotBlocks = F::kSlotBlocks;
+  constexpr int kColumns = F::kWarpColumns;
   extern __shared__ uint8_t raw_smem[];
   uint8_t *base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) & ~uintptr_t(1023));
-  Barriers *bars = reinterpret_cast<Barriers *>(base + kStages * kStageBytes);
+  Barriers *bars = reinterpret_cast<Barriers *>(base + kStages * F::kStageBytes);
   volatile int *abort_flag = &bars->abort_flag;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nb = K / kBlock;
   const int iters = (nb + kStageBlocks - 1) / kStageBlocks;
-  const int m0 = blockIdx.y * kTileM, n0 = blockIdx.x * kTileN;
 
   if (tid == 0) {
     for (int i = 0; i < kStages; ++i) {
       mbar_init(&bars->full[i], 1);
       mbar_init(&bars->empty[i], 1 + kEpilogueWarps);
     }
-    for (int i = 0; i < kTmemBuffers; ++i) {
+    for (int i = 0; i < kSlots; ++i) {
       mbar_init(&bars->tfull[i], 1);
       mbar_init(&bars->tempty[i], kEpilogueWarps);
     }
@@ -173,62 +198,77 @@ gemm_q8_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 
   if (warp == 0) {
     // ---- loader ---------------------------------------------------------------------------
-    if (lane == 0) {
-      int issued = 0;
-      for (int it = 0; it < iters; ++it) {
-        const int s = it % kStages;
-        if (it >= kStages && !mbar_wait(&bars->empty[s], ((it / kStages) - 1) & 1, abort_flag, spin_limit))
-          break;
-        uint8_t *stage = base + s * kStageBytes;
-        mbar_expect_tx(&bars->full[s], kOperandBytes + kOperandBytesB + F::kScaleBytesA + F::kScaleBytesB);
-        issued = it + 1;
-        if (fault == 1 && it == 0)
-          continue;
-        const int k0 = it * kStageK, kb0 = it * kStageBlocks;
-        tma_load_2d(stage, &map_a, k0, m0, &bars->full[s]);
-        tma_load_2d(stage + kOperandBytes, &map_b, k0, n0, &bars->full[s]);
-        tma_load_2d(stage + kOperandBytes + kOperandBytesB, &map_as, m0, kb0, &bars->full[s]);
-        tma_load_2d(stage + kOperandBytes + kOperandBytesB + F::kScaleBytesA, &map_bs, n0, kb0, &bars->full[s]);
+    if (elect_one()) {
+      int use = 0; // stages requested so far, over all tiles of this CTA
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+        const int m0 = (tile % m_tiles) * kTileM, n0 = (tile / m_tiles) * TN;
+        for (int it = 0; it < iters; ++it, ++use) {
+          const int s = use % kStages;
+          if (use >= kStages && !mbar_wait(&bars->empty[s], (use / kStages - 1) & 1, abort_flag, spin_limit)) {
+            ok = false;
+            break;
+          }
+          uint8_t *stage = base + s * F::kStageBytes;
+          mbar_expect_tx(&bars->full[s], F::kCopied);
+          if (fault == 1 && use == 0)
+            continue;
+          const int k0 = it * F::kStageK, kb0 = it * kStageBlocks;
+          tma_load_2d(stage, &map_a, k0, m0, &bars->full[s]);
+          tma_load_2d(stage + kOperandBytes, &map_b, k0, n0, &bars->full[s]);
+          tma_load_2d(stage + kOperandBytes + F::kOperandBytesB, &map_as, m0, kb0, &bars->full[s]);
+          tma_load_2d(stage + kOperandBytes + F::kOperandBytesB + F::kScaleBytesA, &map_bs, n0, kb0, &bars->full[s]);
+        }
       }
       // Leaving after a failed wait: the copies already requested still write into this CTA's
       // shared memory, so each of them gets one more bounded wait before the CTA may exit.
       if (*abort_flag) {
-        for (int it = max(0, issued - kStages); it < issued; ++it)
-          if (!(fault == 1 && it == 0))
-            mbar_wait_quiet(&bars->full[it % kStages], (it / kStages) & 1, spin_limit);
+        for (int i = max(0, use - kStages); i < use; ++i)
+          if (!(fault == 1 && i == 0))
+            mbar_wait_quiet(&bars->full[i % kStages], (i / kStages) & 1, spin_limit);
       }
     }
   } else if (warp == 1) {
     // ---- MMA issue ------------------------------------------------------------------------
-    if (lane == 0) {
-      bool ok = true;
-      for (int it = 0; it < iters && ok; ++it) {
-        const int s = it % kStages;
-        ok = mbar_wait(&bars->full[s], (it / kStages) & 1, abort_flag, spin_limit);
-        if (!ok)
-          break;
-        tc_fence_after();
-        const uint32_t a_addr = smem_u32(base + s * kStageBytes), b_addr = a_addr + kOperandBytes;
-        const int blocks = min(kStageBlocks, nb - it * kStageBlocks);
-        for (int j = 0; j < blocks; ++j) {
-          const int kb = it * kStageBlocks + j;
-          const int buf = kb % kTmemBuffers, use = kb / kTmemBuffers;
-          if (use > 0) {
-            ok = mbar_wait(&bars->tempty[buf], (use - 1) & 1, abort_flag, spin_limit);
-            if (!ok)
+    if (elect_one()) {
+      Ring stages, slots;
+      bool ok = true, reused = false; // reused: every slot has been filled once
+      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+        for (int it = 0; it < iters && ok; ++it) {
+          ok = mbar_wait(&bars->full[stages.at], stages.parity, abort_flag, spin_limit);
+          if (!ok)
+            break;
+          tc_fence_after();
+          const uint64_t a = operand_descriptor(smem_u32(base + stages.at * F::kStageBytes));
+          const uint64_t b = operand_descriptor(smem_u32(base + stages.at * F::kStageBytes) + kOperandBytes);
+          const int blocks = min(kStageBlocks, nb - it * kStageBlocks);
+#pragma unroll
+          for (int j = 0; j < kStageBlocks; ++j) { // descriptors advance in units of 16 bytes
+            if (j >= blocks)
               break;
-            tc_fence_after();
+            if (j % kSlotBlocks == 0 && reused) {
+              ok = mbar_wait(&bars->tempty[slots.at], slots.parity ^ 1, abort_flag, spin_limit);
+              if (!ok)
+                break;
+              tc_fence_after();
+            }
+            const uint32_t d = tmem_base + (slots.at * kSlotBlocks + j % kSlotBlocks) * TN;
+            if (F16) { // two K = 16 instructions per block: the first overwrites, the second accumulates
+              mma_f16(d, a + j * 4, b + j * 4, 0u, Instruction<TN>::kF16);
+              mma_f16(d, a + j * 4 + 2, b + j * 4 + 2, 1u, Instruction<TN>::kF16);
+            } else {
+              mma_i8(d, a + j * 2, b + j * 2, Instruction<TN>::kI8);
+            }
+            if (j % kSlotBlocks == kSlotBlocks - 1 || j == blocks - 1) {
+              mma_commit(&bars->tfull[slots.at]);
+              slots.next(kSlots);
+              reused = reused || slots.at == 0;
+            }
           }
-          const uint32_t d = tmem_base + buf * kTileN;
-          if (F16) { // two K = 16 instructions per block: the first overwrites, the second accumulates
-            mma_f16(d, operand_descriptor(a_addr + j * 64), operand_descriptor(b_addr + j * 64), 0u, Instruction<TN>::kF16);
-            mma_f16(d, operand_descriptor(a_addr + j * 64 + 32), operand_descriptor(b_addr + j * 64 + 32), 1u, Instruction<TN>::kF16);
-          } else {
-            mma_i8(d, operand_descriptor(a_addr + j * 32), operand_descriptor(b_addr + j * 32), Instruction<TN>::kI8);
-          }
-          mma_commit(&bars->tfull[buf]);
+          if (ok)
+            mma_commit(&bars->empty[stages.at]);
+          stages.next(kStages);
         }
-        mma_commit(&bars->empty[s]);
       }
       // A commit's arrival is asynchronous, and nothing else waits for the last ones on `empty`: the
       // CTA must not end (and hand its shared memory to the next CTA on this SM, possibly of another
@@ -239,102 +279,96 @@ gemm_q8_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     }
   } else {
     // ---- epilogue ---------------------------------------------------------------------------
-    const int quarter = warp & 3;                  // tensor-memory lanes 32*quarter .. +31 (fixed by the warp number)
-    const int colq = (warp - kEpilogueWarp0) >> 2; // columns kWarpColumns * colq .. + kWarpColumns - 1
+    const int quarter = warp & 3;                                  // tensor-memory lanes 32 * quarter .. + 31 (fixed by the warp number)
+    const int column0 = ((warp - kEpilogueWarp0) >> 2) * kColumns; // this warp's columns of the tile
     const int row = quarter * 32 + lane;
-    const int gm = m0 + row;
-    float acc[kWarpColumns];
+    const uint32_t taddr0 = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + column0;
+    Ring stages, slots;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+      const int gm = (tile % m_tiles) * kTileM + row, gn0 = (tile / m_tiles) * TN + column0;
+      float acc[kColumns];
 #pragma unroll
-    for (int c = 0; c < kWarpColumns; ++c)
-      acc[c] = 0.0f;
-    bool ok = true;
-    for (int kb = 0; kb < nb && ok; ++kb) {
-      const int buf = kb % kTmemBuffers;
-      ok = __all_sync(0xffffffffu, mbar_wait(&bars->tfull[buf], (kb / kTmemBuffers) & 1, abort_flag, spin_limit));
-      if (!ok) // the whole warp leaves together: the tensor-memory loads below are warp-wide
-        break;
-      tc_fence_after();
-      const int it = kb / kStageBlocks, s = it % kStages, j = kb % kStageBlocks;
-      // The stage's scales arrived with the operands; observing the stage's own barrier (long
-      // complete by now) is what makes the copied bytes visible to these loads.
-      if (j == 0 && !__all_sync(0xffffffffu, mbar_wait(&bars->full[s], (it / kStages) & 1, abort_flag, spin_limit))) {
-        ok = false;
-        break;
-      }
-      const float *scales = reinterpret_cast<const float *>(base + s * kStageBytes + kOperandBytes + kOperandBytesB);
-      const float a_scale = scales[j * kTileM + row];
-      const float4 *w_scale = reinterpret_cast<const float4 *>(scales + kStageBlocks * kTileM + j * kTileN + colq * kWarpColumns);
-      uint32_t raw[kWarpColumns];
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * kTileN + colq * kWarpColumns;
-      if (kWarpColumns == 32) {
-        tmem_load32(taddr, *reinterpret_cast<uint32_t(*)[32]>(raw));
-      } else { // 32 + 8 columns, one wait for both loads
-        tmem_issue32(taddr, *reinterpret_cast<uint32_t(*)[32]>(raw));
-        tmem_issue8(taddr + 32, *reinterpret_cast<uint32_t(*)[8]>(raw + 32));
-        tmem_wait_loads();
-      }
-      // The buffer is handed back before any arithmetic, so that the MMA of a later block can
-      // reuse it while this one is still being folded in.
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0)
-        mbar_arrive(&bars->tempty[buf]);
-      float v[kWarpColumns];
+      for (int c = 0; c < kColumns; ++c)
+        acc[c] = 0.0f;
+      bool ok = true;
+      for (int it = 0; it < iters; ++it) {
+        // The stage's scales arrived with the operands; observing the stage's own barrier (long
+        // complete by now) is what makes the copied bytes visible to these loads.
+        ok = warp_wait(&bars->full[stages.at], stages.parity, abort_flag, spin_limit);
+        if (!ok) // the whole warp leaves together: the tensor-memory loads below are warp-wide
+          break;
+        const float *scales = reinterpret_cast<const float *>(base + stages.at * F::kStageBytes + kOperandBytes + F::kOperandBytesB);
+        const int blocks = min(kStageBlocks, nb - it * kStageBlocks);
 #pragma unroll
-      for (int u = 0; u < kWarpColumns; ++u)
-        v[u] = F16 ? __uint_as_float(raw[u]) : __int2float_rn(static_cast<int>(raw[u]));
-#pragma unroll
-      for (int g = 0; g < kWarpColumns / 4; ++g) {
-        const float4 w4 = w_scale[g];
-        if (PACKED) {
-          float f0, f1, f2, f3;
-          mul2(f0, f1, a_scale, a_scale, w4.x, w4.y);
-          mul2(f2, f3, a_scale, a_scale, w4.z, w4.w);
-          fma2(acc[g * 4 + 0], acc[g * 4 + 1], v[g * 4 + 0], v[g * 4 + 1], f0, f1);
-          fma2(acc[g * 4 + 2], acc[g * 4 + 3], v[g * 4 + 2], v[g * 4 + 3], f2, f3);
-        } else {
-          acc[g * 4 + 0] = __fmaf_rn(v[g * 4 + 0], __fmul_rn(a_scale, w4.x), acc[g * 4 + 0]);
-          acc[g * 4 + 1] = __fmaf_rn(v[g * 4 + 1], __fmul_rn(a_scale, w4.y), acc[g * 4 + 1]);
-          acc[g * 4 + 2] = __fmaf_rn(v[g * 4 + 2], __fmul_rn(a_scale, w4.z), acc[g * 4 + 2]);
-          acc[g * 4 + 3] = __fmaf_rn(v[g * 4 + 3], __fmul_rn(a_scale, w4.w), acc[g * 4 + 3]);
-        }
-      }
-      if (DOTS) {
-        if (gm < M) {
-#pragma unroll
-          for (int u = 0; u < kWarpColumns; ++u) {
-            const int gn = n0 + colq * kWarpColumns + u;
-            if (gn < N)
-              dots_out[(static_cast<size_t>(gm) * N + gn) * nb + kb] = F16 ? __float2int_rn(v[u]) : static_cast<int>(raw[u]);
+        for (int j = 0; j < kStageBlocks; ++j) {
+          if (j >= blocks)
+            break;
+          if (j % kSlotBlocks == 0) {
+            ok = warp_wait(&bars->tfull[slots.at], slots.parity, abort_flag, spin_limit);
+            if (!ok)
+              break;
+            tc_fence_after();
           }
-        }
-      }
-      if (j == kStageBlocks - 1 || kb == nb - 1) { // done with this stage's scales
-        __syncwarp();
-        if (lane == 0)
-          mbar_arrive(&bars->empty[s]);
-      }
-    }
-    if (ok && gm < M) {
+          uint32_t raw[kColumns];
+          tmem_load_columns<kColumns>(taddr0 + (slots.at * kSlotBlocks + j % kSlotBlocks) * TN, raw);
+          if (j % kSlotBlocks == kSlotBlocks - 1 || j == blocks - 1) {
+            // The slot is handed back before its last block is folded in.
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0)
+              mbar_arrive(&bars->tempty[slots.at]);
+            slots.next(kSlots);
+          }
+          const float a_scale = scales[j * kTileM + row];
+          const float4 *w_scale = reinterpret_cast<const float4 *>(scales + kStageBlocks * kTileM + j * TN + column0);
 #pragma unroll
-      for (int g = 0; g < kWarpColumns / 8; ++g) {
-        const int gn = n0 + colq * kWarpColumns + g * 8;
-        if (gn < N) { // N is a multiple of 8, so a group of eight is entirely inside or outside
-          float o[8];
-#pragma unroll
-          for (int u = 0; u < 8; ++u)
-            o[u] = apply_activation(acc[g * 8 + u], activation);
-          if (y_dtype == kBF16) {
-            uint32_t packed[4];
+          for (int g = 0; g < kColumns / 4; ++g) {
+            const float4 w = w_scale[g];
+            float v[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u)
-              packed[u] = static_cast<uint32_t>(f32_to_bf16(o[2 * u])) | (static_cast<uint32_t>(f32_to_bf16(o[2 * u + 1])) << 16);
-            *reinterpret_cast<uint4 *>(static_cast<uint16_t *>(y) + static_cast<size_t>(gm) * N + gn) =
-                make_uint4(packed[0], packed[1], packed[2], packed[3]);
-          } else {
-            float4 *dst = reinterpret_cast<float4 *>(static_cast<float *>(y) + static_cast<size_t>(gm) * N + gn);
-            dst[0] = make_float4(o[0], o[1], o[2], o[3]);
-            dst[1] = make_float4(o[4], o[5], o[6], o[7]);
+              v[u] = F16 ? __uint_as_float(raw[4 * g + u]) : __int2float_rn(static_cast<int>(raw[4 * g + u]));
+            fold2(acc[4 * g + 0], acc[4 * g + 1], v[0], v[1], a_scale, w.x, w.y);
+            fold2(acc[4 * g + 2], acc[4 * g + 3], v[2], v[3], a_scale, w.z, w.w);
+            if (DOTS && gm < M) {
+#pragma unroll
+              for (int u = 0; u < 4; ++u)
+                if (gn0 + 4 * g + u < N)
+                  dots_out[(static_cast<size_t>(gm) * N + gn0 + 4 * g + u) * nb + it * kStageBlocks + j] =
+                      F16 ? __float2int_rn(v[u]) : static_cast<int>(raw[4 * g + u]);
+            }
+          }
+        }
+        if (!ok)
+          break;
+        __syncwarp();
+        if (lane == 0) // done with this stage's scales
+          mbar_arrive(&bars->empty[stages.at]);
+        stages.next(kStages);
+      }
+      if (!ok)
+        break;
+      if (gm < M) {
+#pragma unroll
+        for (int g = 0; g < kColumns / 8; ++g) {
+          const int gn = gn0 + g * 8;
+          if (gn < N) { // N is a multiple of 8, so a group of eight is entirely inside or outside
+            float o[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+              o[u] = apply_activation(acc[g * 8 + u], activation);
+            if (y_dtype == kBF16) {
+              uint32_t packed[4];
+#pragma unroll
+              for (int u = 0; u < 4; ++u)
+                packed[u] = static_cast<uint32_t>(f32_to_bf16(o[2 * u])) | (static_cast<uint32_t>(f32_to_bf16(o[2 * u + 1])) << 16);
+              *reinterpret_cast<uint4 *>(static_cast<uint16_t *>(y) + static_cast<size_t>(gm) * N + gn) =
+                  make_uint4(packed[0], packed[1], packed[2], packed[3]);
+            } else {
+              float4 *dst = reinterpret_cast<float4 *>(static_cast<float *>(y) + static_cast<size_t>(gm) * N + gn);
+              dst[0] = make_float4(o[0], o[1], o[2], o[3]);
+              dst[1] = make_float4(o[4], o[5], o[6], o[7]);
+            }
           }
         }
       }
@@ -390,83 +424,76 @@ __global__ void weights_to_f16_kernel(const int8_t *__restrict__ wq, const uint1
   }
 }
 
-// rows x K operand plane, K contiguous: boxes of 128 rows x 128 bytes of K (64 f16 or 128 int8),
-// 128-byte swizzle; out-of-range parts read as zero.
-bool operand_map(CUtensorMap *map, const void *plane, int64_t rows, int K, bool f16, int box_rows = kTileM) {
-  EncodeTiled encode = encode_tiled();
-  if (!encode)
-    return false;
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(K) * (f16 ? 2 : 1)};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(f16 ? 64 : 128), static_cast<cuuint32_t>(box_rows)};
-  const cuuint32_t elem[2] = {1, 1};
-  return encode(map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(plane), dims,
-                strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
+struct GemmCall {
+  const void *a;
+  const float *ast;
+  int M, K;
+  const void *w;
+  const float *wst;
+  int N;
+  void *y;
+  int y_dtype, activation;
+  int32_t *dots_out;
+  int *error_flag;
+  cudaStream_t stream;
+  uint32_t spin_limit;
+  int fault, sm_count;
+};
 
-// nb x ld f32, block-major: boxes of a stage's blocks x 128 entries.
-bool scale_map(CUtensorMap *map, const void *plane, int64_t entries, int64_t ld, int nb, int stage_blocks, int box_entries = kTileM) {
-  EncodeTiled encode = encode_tiled();
-  if (!encode)
-    return false;
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(entries), static_cast<cuuint64_t>(nb)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 4};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(box_entries), static_cast<cuuint32_t>(stage_blocks)};
-  const cuuint32_t elem[2] = {1, 1};
-  return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void *>(plane), dims, strides, box, elem,
-                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-template <bool F16, bool PACKED, int TN>
-cudaError_t launch_tile(const void *a, const float *ast, int M, int K, const void *w, const float *wst, int N, void *y,
-                        int y_dtype, int activation, int32_t *dots_out, int *error_flag, cudaStream_t stream, uint32_t spin_limit,
-                        int fault) {
+template <bool F16, int TN> cudaError_t launch_tile(const GemmCall &c) {
   using F = Form<F16, TN>;
-  const int nb = K / kBlock;
+  const int nb = c.K / kBlock;
   CUtensorMap map_a, map_b, map_as, map_bs;
-  if (!operand_map(&map_a, a, M, K, F16) || !operand_map(&map_b, w, N, K, F16, TN) ||
-      !scale_map(&map_as, ast, M, gemm_tc16_scale_pitch(M), nb, F::kStageBlocks) ||
-      !scale_map(&map_bs, wst, N, N, nb, F::kStageBlocks, TN))
+  if (!gemm_operand_map(&map_a, c.a, c.M, c.K, F16, kTileM) || !gemm_operand_map(&map_b, c.w, c.N, c.K, F16, TN) ||
+      !gemm_scale_map(&map_as, c.ast, c.M, gemm_tc16_scale_pitch(c.M), nb, F::kStageBlocks, kTileM) ||
+      !gemm_scale_map(&map_bs, c.wst, c.N, c.N, nb, F::kStageBlocks, TN))
     return cudaErrorNotSupported;
-  const void *kernel = dots_out ? reinterpret_cast<const void *>(gemm_q8_tma_kernel<F16, PACKED, true, TN>)
-                                : reinterpret_cast<const void *>(gemm_q8_tma_kernel<F16, PACKED, false, TN>);
-  if (cudaError_t e = opt_in_shared_memory(kernel, F::kSmemBytes); e != cudaSuccess)
+  auto kernel = c.dots_out ? gemm_q8_tma_kernel<F16, true, TN> : gemm_q8_tma_kernel<F16, false, TN>;
+  if (cudaError_t e = opt_in_shared_memory(reinterpret_cast<const void *>(kernel), F::kSmemBytes); e != cudaSuccess)
     return e;
-  dim3 grid((N + TN - 1) / TN, (M + kTileM - 1) / kTileM);
-  if (dots_out)
-    launch_chained(gemm_q8_tma_kernel<F16, PACKED, true, TN>, grid, dim3(kThreads), F::kSmemBytes, stream, map_a, map_b, map_as,
-                   map_bs, M, K, N, y, y_dtype, activation, dots_out, error_flag, spin_limit, fault);
-  else
-    launch_chained(gemm_q8_tma_kernel<F16, PACKED, false, TN>, grid, dim3(kThreads), F::kSmemBytes, stream, map_a, map_b, map_as,
-                   map_bs, M, K, N, y, y_dtype, activation, dots_out, error_flag, spin_limit, fault);
+  const int m_tiles = (c.M + kTileM - 1) / kTileM;
+  const int64_t tiles = static_cast<int64_t>(m_tiles) * ((c.N + TN - 1) / TN);
+  if (tiles >= (1 << 30))
+    return cudaErrorInvalidValue;
+  launch_chained(kernel, dim3(static_cast<unsigned>(std::min<int64_t>(tiles, c.sm_count))), dim3(kThreads), F::kSmemBytes, c.stream,
+                 map_a, map_b, map_as, map_bs, c.M, c.K, c.N, static_cast<int>(tiles), m_tiles, c.y, c.y_dtype, c.activation,
+                 c.dots_out, c.error_flag, c.spin_limit, c.fault);
   return cudaGetLastError();
 }
 
-// Tile width for an M x N output: every wave of tiles costs about the same whatever it holds, a
-// 160-wide tile a quarter more than a 128-wide one; LLMCP_B200_GEMM_TILE=128|160 overrides.
-int choose_tile(int M, int N) {
+// LLMCP_B200_GEMM_TILE=64|96|128: the tile width for every shape, few rows included; 0 = not set.
+int forced_tile() {
   const char *flag = std::getenv("LLMCP_B200_GEMM_TILE");
   const int forced = flag ? std::atoi(flag) : 0;
-  if (forced == 128 || forced == 160)
-    return forced;
-  int sm_count = 148;
-  if (current_sm_count(&sm_count) != cudaSuccess || sm_count <= 0)
-    sm_count = 148;
-  const int64_t sms = sm_count;
-  const int64_t rows = (M + kTileM - 1) / kTileM;
-  const int64_t waves128 = (rows * ((N + 127) / 128) + sms - 1) / sms, waves160 = (rows * ((N + 159) / 160) + sms - 1) / sms;
-  return waves160 * 5 < waves128 * 4 ? 160 : 128;
+  return forced == 64 || forced == 96 || forced == 128 ? forced : 0;
 }
 
-template <bool F16, bool PACKED>
-cudaError_t launch_form(const void *a, const float *ast, int M, int K, const void *w, const float *wst, int N, void *y,
-                        int y_dtype, int activation, int32_t *dots_out, int *error_flag, cudaStream_t stream, uint32_t spin_limit,
-                        int fault) {
-  if (choose_tile(M, N) == 160)
-    return launch_tile<F16, PACKED, 160>(a, ast, M, K, w, wst, N, y, y_dtype, activation, dots_out, error_flag, stream, spin_limit, fault);
-  return launch_tile<F16, PACKED, 128>(a, ast, M, K, w, wst, N, y, y_dtype, activation, dots_out, error_flag, stream, spin_limit, fault);
+// Tile width for an M x N output: a CTA works through ceil(tiles / SMs) tiles, each at a cost that grows with its
+// width and has a part that does not (the hand-off of a block, worth about 72 columns: 23.4, 27.8 and
+// 33.7 us for one tile of K = 2560).
+int choose_tile(int M, int N, int sm_count) {
+  if (const int forced = forced_tile())
+    return forced;
+  const int64_t rows = (M + kTileM - 1) / kTileM;
+  int best = 128;
+  int64_t best_cost = INT64_MAX;
+  for (const int width : {128, 96, 64}) {
+    const int64_t tiles = rows * ((N + width - 1) / width), cost = (tiles + sm_count - 1) / sm_count * (width + 72);
+    if (cost < best_cost)
+      best = width, best_cost = cost;
+  }
+  return best;
+}
+
+template <bool F16> cudaError_t launch_form(const GemmCall &c) {
+  switch (choose_tile(c.M, c.N, c.sm_count)) {
+  case 64:
+    return launch_tile<F16, 64>(c);
+  case 96:
+    return launch_tile<F16, 96>(c);
+  default:
+    return launch_tile<F16, 128>(c);
+  }
 }
 
 // [rows][K/32] scales -> block-major f32 [K/32][ld]; scales are f32 (activations) or f16 bits (weights).
@@ -511,16 +538,19 @@ cudaError_t launch_gemm_q8_tma(int form, const void *a, const float *ast, int M,
   if (M <= 0 || N % 8 != 0 || K % kBlock != 0)
     return cudaErrorInvalidValue;
   if (spin_limit == 0)
-    spin_limit = 1u << 26; // about a second
+    spin_limit = tc::kSpinLimit;
+  GemmCall call = {a, ast, M, K, w, wst, N, y, y_dtype, activation, dots_out, error_flag, stream, spin_limit, fault, 148};
+  int sms = 0;
+  if (current_sm_count(&sms) == cudaSuccess && sms > 0)
+    call.sm_count = sms;
   switch (form) {
   case kGemmF16:
-    return launch_form<true, false>(a, ast, M, K, w, wst, N, y, y_dtype, activation, dots_out, error_flag, stream, spin_limit, fault);
   case kGemmF16Packed:
-    return launch_form<true, true>(a, ast, M, K, w, wst, N, y, y_dtype, activation, dots_out, error_flag, stream, spin_limit, fault);
+    return launch_form<true>(call);
   case kGemmI8:
-    return launch_form<false, false>(a, ast, M, K, w, wst, N, y, y_dtype, activation, dots_out, error_flag, stream, spin_limit, fault);
+    return launch_form<false>(call);
   case kGemmI8Packed:
-    return launch_form<false, true>(a, ast, M, K, w, wst, N, y, y_dtype, activation, dots_out, error_flag, stream, spin_limit, fault);
+    return launch_form<false>(call);
   default:
     return cudaErrorInvalidValue;
   }

@@ -15,6 +15,13 @@ namespace tc {
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
+// True in one lane of the (converged) warp; the compiler knows that a single lane runs what it guards.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t elected;
+  asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(elected));
+  return elected != 0;
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
@@ -26,19 +33,28 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
                : "memory");
 }
 
+// One bounded look at the phase with the given parity: the hardware may suspend the thread for up to kPollNs.  Without
+// the hint a poll returns after some 20 cycles, and the single lanes that wait most of the time (loader, MMA issue)
+// then took a third of an SM's issue slots and its instruction cache from the warps that compute.
+constexpr uint32_t kPollNs = 1000;
+constexpr uint32_t kSpinLimit = 1u << 21; // polls before a wait gives up, unless the caller says otherwise: seconds
+__device__ __forceinline__ bool mbar_poll(uint32_t addr, uint32_t parity) {
+  uint32_t done;
+  asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }"
+               : "=r"(done)
+               : "r"(addr), "r"(parity), "r"(kPollNs)
+               : "memory");
+  return done != 0;
+}
+
 // Waits for the phase with the given parity; gives up when `abort_flag` is raised or after `limit`
 // polls (and then raises it).  Returns false on failure.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag, uint32_t limit) {
   const uint32_t addr = smem_u32(bar);
   for (uint32_t spin = 0; spin < limit; ++spin) {
-    uint32_t done;
-    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-                 : "=r"(done)
-                 : "r"(addr), "r"(parity)
-                 : "memory");
-    if (done)
+    if (mbar_poll(addr, parity))
       return true;
-    if ((spin & 63) == 63 && *abort_flag)
+    if (*abort_flag)
       return false;
   }
   *abort_flag = 1;
@@ -48,15 +64,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
 // The same wait without the abort protocol (used while leaving after an abort).
 __device__ __forceinline__ bool mbar_wait_quiet(uint64_t *bar, uint32_t parity, uint32_t limit) {
   const uint32_t addr = smem_u32(bar);
-  for (uint32_t spin = 0; spin < limit; ++spin) {
-    uint32_t done;
-    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-                 : "=r"(done)
-                 : "r"(addr), "r"(parity)
-                 : "memory");
-    if (done)
+  for (uint32_t spin = 0; spin < limit; ++spin)
+    if (mbar_poll(addr, parity))
       return true;
-  }
   return false;
 }
 
@@ -112,6 +122,13 @@ __device__ __forceinline__ void tmem_issue32(uint32_t taddr, uint32_t (&r)[32]) 
       : "r"(taddr)
       : "memory");
 }
+__device__ __forceinline__ void tmem_issue16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+                 "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+               : "r"(taddr)
+               : "memory");
+}
 __device__ __forceinline__ void tmem_issue8(uint32_t taddr, uint32_t (&r)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
@@ -145,6 +162,35 @@ inline EncodeTiled encode_tiled() {
       fn = reinterpret_cast<EncodeTiled>(p);
   }
   return fn;
+}
+
+// rows x K operand plane, K contiguous: boxes of box_rows rows x 128 bytes of K (64 f16 or 128 int8),
+// 128-byte swizzle; out-of-range parts read as zero.
+inline bool gemm_operand_map(CUtensorMap *map, const void *plane, int64_t rows, int K, bool f16, int box_rows) {
+  EncodeTiled encode = encode_tiled();
+  if (!encode)
+    return false;
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(K) * (f16 ? 2 : 1)};
+  const cuuint32_t box[2] = {static_cast<cuuint32_t>(f16 ? 64 : 128), static_cast<cuuint32_t>(box_rows)};
+  const cuuint32_t elem[2] = {1, 1};
+  return encode(map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(plane), dims,
+                strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// nb x ld f32, block-major: boxes of a stage's blocks x box_entries entries.
+inline bool gemm_scale_map(CUtensorMap *map, const void *plane, int64_t entries, int64_t ld, int nb, int stage_blocks, int box_entries) {
+  EncodeTiled encode = encode_tiled();
+  if (!encode)
+    return false;
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(entries), static_cast<cuuint64_t>(nb)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 4};
+  const cuuint32_t box[2] = {static_cast<cuuint32_t>(box_entries), static_cast<cuuint32_t>(stage_blocks)};
+  const cuuint32_t elem[2] = {1, 1};
+  return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void *>(plane), dims, strides, box, elem,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 } // namespace tc

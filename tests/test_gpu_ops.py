@@ -517,3 +517,20 @@ def test_linear_q8_both_tile_widths(monkeypatch):
     assert np.array_equal(y.view(np.uint32), oracle.linear_q8(x, packed, N, y_bf16=False).view(np.uint32))
     assert np.array_equal(dots, oracle.block_dots(oracle.act_quant(x)[0], packed, N))
 
+
+
+@pytest.mark.parametrize("tile", ["64", "96", "128"])
+@pytest.mark.parametrize("M,N,K", [(130, 264, 2560), (1000, 2568, 96), (3, 8, 32), (520, 8200, 32)])
+def test_gemm_tma_tile_widths(monkeypatch, tile, M, N, K):
+    """Every tile width of the tcgen05 GEMM, both operand forms: partial tiles, several tiles per CTA, an odd number of
+    blocks (the last hand-off holds one)."""
+    torch = pytest.importorskip("torch")
+    lib, stream, ptr, planes, want = _tma_gemm_setup(torch, M, N, K, M + N + K + 1)
+    monkeypatch.setenv("LLMCP_B200_GEMM_TILE", tile)
+    for form in (1, 3):
+        status = torch.zeros(1, dtype=torch.int32, device="cuda")
+        y = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
+        _tma_gemm(lib, stream, ptr, planes, form, M, N, K, y, status)
+        torch.cuda.synchronize()
+        assert int(status.item()) == 0
+        assert np.array_equal(y.cpu().numpy().view(np.uint32), want.view(np.uint32)), form
