@@ -550,6 +550,9 @@ cudaError_t launch_gemm_q8_tma(int form, const void *a, const float *ast, int M,
   case kGemmI8:
     return launch_form<false>(call);
   case kGemmI8Packed:
+    if (!forced_tile() && gemm_few_preferred(M, N, call.sm_count))
+      return launch_gemm_q8_few(static_cast<const int8_t *>(a), ast, M, K, static_cast<const int8_t *>(w), wst, N, y, y_dtype,
+                                activation, dots_out, error_flag, stream, spin_limit, fault);
     return launch_form<false>(call);
   default:
     return cudaErrorInvalidValue;

@@ -100,6 +100,12 @@ void launch_scales_block_major(const void *scales, int scales_are_f16, int64_t r
 cudaError_t launch_gemm_q8_tma(int form, const void *a, const float *ast, int M, int K, const void *w, const float *wst, int N,
                                void *y, int y_dtype, int activation, int32_t *dots_out, int *error_flag, cudaStream_t stream,
                                uint32_t spin_limit = 0, int fault = 0);
+// The same contraction in narrow tiles (gemm_few.cu); operands as for kGemmI8Packed, which takes this form by itself
+// where gemm_few_preferred.
+bool gemm_few_preferred(int M, int N, int sm_count);
+cudaError_t launch_gemm_q8_few(const int8_t *aq, const float *ast, int M, int K, const int8_t *wq, const float *wst, int N,
+                               void *y, int y_dtype, int activation, int32_t *dots_out, int *error_flag, cudaStream_t stream,
+                               uint32_t spin_limit, int fault);
 // status (device int, optional): bit 1 is raised when a token id lies outside [0, vocab); such a
 // row is written as zeros and the table is not read.
 // Second form of the tensor-core GEMM (gemm_tma.cu): the int8 operands held as f16 values and the

@@ -519,6 +519,43 @@ def test_linear_q8_both_tile_widths(monkeypatch):
 
 
 
+@pytest.mark.parametrize("M,N,K", [(2, 8, 32), (32, 16, 2560), (33, 72, 96), (64, 2568, 288), (65, 136, 160), (7, 9216, 128),
+                                   (128, 2560, 4096), (300, 32, 2560), (1024, 40, 608), (64, 38016, 64), (40, 4104, 544)])
+def test_gemm_few_rows(M, N, K):
+    """The narrow-tile form of the default GEMM: bit-identical to the oracle at the edges of its tiles (16, 32 and 64
+    weight rows, 32 and 64 rows), with a last stage that is not full, over several tiles per CTA, f32 and bf16 out."""
+    import ctypes as C
+    torch = pytest.importorskip("torch")
+    lib, stream, ptr, planes, want = _tma_gemm_setup(torch, M, N, K, M + N + K)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    y = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
+    _tma_gemm(lib, stream, ptr, planes, 1, M, N, K, y, status)
+    yb = torch.zeros((M, N), dtype=torch.bfloat16, device="cuda")
+    assert lib.llmcp_dev_gemm_q8_tma(1, ptr(planes["aq"]), ptr(planes["ast"]), C.c_int64(M), C.c_int64(K), ptr(planes["wq"]),
+                                     ptr(planes["wst"]), C.c_int64(N), ptr(yb), 1, 0, ptr(status), C.c_uint32(0), 0, stream) == 0
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    assert np.array_equal(y.cpu().numpy().view(np.uint32), want.view(np.uint32))
+    assert torch.equal(yb, torch.from_numpy(want).to(torch.bfloat16).cuda())
+
+
+def test_gemm_few_rows_bounded_wait_runs_out_and_recovers():
+    """As for the wide form: the withheld stage ends every wait, nothing is written, the next launch is correct."""
+    torch = pytest.importorskip("torch")
+    M, N, K = 24, 520, 2560
+    lib, stream, ptr, planes, want = _tma_gemm_setup(torch, M, N, K, 98)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    y = torch.full((M, N), 7.0, dtype=torch.float32, device="cuda")
+    _tma_gemm(lib, stream, ptr, planes, 1, M, N, K, y, status, spin_limit=1 << 12, fault=1)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 1 and bool((y == 7.0).all())
+    status.zero_()
+    _tma_gemm(lib, stream, ptr, planes, 1, M, N, K, y, status)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    assert np.array_equal(y.cpu().numpy().view(np.uint32), want.view(np.uint32))
+
+
 @pytest.mark.parametrize("tile", ["64", "96", "128"])
 @pytest.mark.parametrize("M,N,K", [(130, 264, 2560), (1000, 2568, 96), (3, 8, 32), (520, 8200, 32)])
 def test_gemm_tma_tile_widths(monkeypatch, tile, M, N, K):
