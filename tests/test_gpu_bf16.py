@@ -42,6 +42,18 @@ def test_linear_bf16_against_f32_product(M, N, K):
         assert np.abs(got_b - act(want)).max() <= 2.0 ** -7 * max(1.0, np.abs(act(want)).max())  # one bf16 rounding
 
 
+@pytest.mark.parametrize("N,K", [(1, 16), (7, 48), (2, 512), (9, 528), (4737, 2064), (3, 12288)])
+def test_gemv_bf16_edges(N, K):
+    """One row: pieces past the row's end, odd row counts, more rows than warps in flight, the longest row."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(N + K)
+    x, w = bf16(rng.standard_normal((1, K))), bf16(rng.standard_normal((N, K)) * 0.05)
+    want = (torch.from_numpy(f(x)).double() @ torch.from_numpy(f(w)).double().T).numpy()
+    magnitude = np.abs(f(x)).astype(np.float64) @ np.abs(f(w)).astype(np.float64).T
+    # a lane adds K / 32 products and the lanes are added in five steps: |error| <= (K / 32 + 22) 2^-24 sum |x w|
+    assert (np.abs(L.ops.linear_bf16(x, w, y_bf16=False) - want) <= (K / 32 + 22) * 2.0 ** -24 * magnitude).all()
+
+
 def oracle_dims(d):
     return dict(full_interval=d.full_interval, heads=d.heads, kv_heads=d.kv_heads, head_dim=d.head_dim,
                 rotary=d.rotary, lin_k_heads=d.lin_k_heads, lin_v_heads=d.lin_v_heads, lin_k_dim=d.lin_k_dim,
