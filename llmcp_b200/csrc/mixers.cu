@@ -404,57 +404,239 @@ gdn_recurrence_pipelined_kernel(const uint16_t *__restrict__ conv, const float *
   }
 }
 
-// Fast form of the recurrence for calls of more than one token: the same two-tokens-in-flight loop,
-// but a warp owns 8 value columns and each column's 128 state rows are shared by four lanes (32
-// rows each), so the two dependent chains per token are 32 long instead of 128 and end in two
-// shuffles; multiply and add are fused.  What bounds the exact kernel, and still bounds this one, is
-// how fast ONE warp can walk its dependent instructions, so a head is spread over 16 independent
-// warps instead of 4.  A token then takes a few hundred cycles, less than a trip to L2, so the
-// inputs (k, q, decay, beta, the 8 values) arrive by cp.async in chunks of 8 tokens, three chunks in
-// shared memory per warp: the one in use, the next (token t + 1's k is needed beside token t) and
-// the one in flight.  The sums differ from the reference's order (row groups are added as a tree)
-// and from its roundings (fused multiply-adds): results agree with the exact kernels to f32
-// rounding noise, not bit for bit.  Measured with 4 columns and eight lanes per column instead:
-// slower (twice the shared memory per column, so half the CTAs fit).
-// grid (value head, dv / 32), 128 threads: four independent warps that share nothing.
+// The recurrence for calls of more than one token (dk = 128), both modes: the same two-tokens-in-flight loop, but a warp
+// owns 8 value columns and each column's 128 state rows are shared by several lanes, so a layer is 512 warps, one for
+// nearly every scheduler, where one thread per column makes 128.  What bounds it is how fast one warp walks its
+// dependent instructions, and the shared-memory reads of k and q (every lane needs all rows of its part).
+//   exact: four lanes per column, 32 rows each.  The products of a token are formed by all lanes at once; the two serial
+//     sums then go through the lanes in row order, 32 additions in the lane whose rows come next, a shuffle to the
+//     following one.  Every value is produced by the operations of the kernels above in the same order.
+//   fast: eight lanes per pair of columns, 16 rows each, fused multiply-adds two rows at a time; the sums end in a
+//     shuffle tree, so they differ from the exact ones by f32 rounding.  Two columns per lane, because a row of k and q
+//     read from shared memory then serves both.
+// Inputs (k, q, decay, beta, the CTA's 32 values) arrive by cp.async in chunks of 8 tokens shared by the CTA's four
+// warps, three chunks in shared memory: the one in use, the next (token t + 1's k is needed beside token t) and the one
+// in flight.  Row parts stand 16 bytes out of step there, so that the lanes' 16-byte reads fall into different banks.
+// Measured, 32 heads: exact 0.82 -> 0.59 us per token (one thread per column before), fast 0.38 -> 0.27 (four lanes per
+// column, a copy of the inputs per warp).  Two rows per instruction do not help the exact form: the f32 pipe takes
+// them at half the rate, and ptxas makes one fma of a two-row multiply and a two-row add.
+// grid (value head, dv / 32), 128 threads.
 constexpr int kSplitChunk = 8; // tokens per chunk
 constexpr int kSplitWarps = 4;
 constexpr int kSplitCols = 8;  // value columns per warp
-constexpr int kSplitLanes = 32 / kSplitCols; // lanes per column
 
-// A lane reads its 16-byte pieces of k and q at the same offset inside its own row group; the groups
-// are kept 16 bytes out of step (rows + 4 floats apart) so that those reads fall into different banks.
-template <int DK> struct SplitChunk {
-  static constexpr int kRows = DK / kSplitLanes, kPitch = kRows + 4;
-  float kq[kSplitChunk][2][kSplitLanes][kPitch]; // per token: kn and qn, by row group
-  uint16_t value[kSplitChunk][kSplitCols];
+template <int DK, int PARTS> struct SplitChunk {
+  static constexpr int kRows = DK / PARTS, kPitch = kRows + 4;
+  float kq[kSplitChunk][2][PARTS][kPitch]; // per token: kn and qn, by part
+  uint16_t value[kSplitChunk][kSplitWarps * kSplitCols];
   float dc[kSplitChunk], bt[kSplitChunk];
 };
 
-template <int DK>
+// Two f32 values in one 64-bit register pair.
+using Pair = unsigned long long;
+using Pair2 = ulonglong2;
+__device__ __forceinline__ Pair make_pair(float lo, float hi) {
+  Pair p;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(lo), "f"(hi));
+  return p;
+}
+__device__ __forceinline__ float2 unpack(Pair p) {
+  float2 v;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ Pair mul2(Pair a, Pair b) {
+  Pair d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
+  Pair d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+// One lane's rows of its column (exact form).  advance: rows as token t leaves them, o = sum_k s_k q_k; when there is a
+// token t + 1, rows decayed for it and kv = sum_k s_k k'_k.  All lanes of the column return the sums.
+template <int DK> struct ExactColumn {
+  static constexpr int kParts = 4, kRows = DK / kParts, kLanes = 32 / kParts;
+  float s[kRows];
+
+  __device__ __forceinline__ void load(const float *col, int64_t dv) {
+#pragma unroll
+    for (int k = 0; k < kRows; ++k)
+      s[k] = col[k * dv];
+  }
+  __device__ __forceinline__ void store(float *col, int64_t dv) const {
+#pragma unroll
+    for (int k = 0; k < kRows; ++k)
+      col[k * dv] = s[k];
+  }
+  // The serial sum over the column's rows: after step p every lane holds the sum over parts 0 .. p.
+  template <bool TWO> static __device__ __forceinline__ void sums(const float (&po)[kRows], const float (&pk)[kRows], int c, float &o, float &kv) {
+    o = 0.0f, kv = 0.0f;
+#pragma unroll
+    for (int p = 0; p < kParts; ++p) {
+#pragma unroll
+      for (int k = 0; k < kRows; ++k) {
+        kv = __fadd_rn(kv, pk[k]);
+        if (TWO)
+          o = __fadd_rn(o, po[k]);
+      }
+      kv = __shfl_sync(0xffffffffu, kv, p * kLanes + c);
+      if (TWO)
+        o = __shfl_sync(0xffffffffu, o, p * kLanes + c);
+    }
+  }
+  __device__ __forceinline__ float first(const float *kn, float dc, int c) { // token 0: decay and first sum on their own
+    float pk[kRows], o, kv;
+#pragma unroll
+    for (int k4 = 0; k4 < kRows; k4 += 4) {
+      const float4 kk = *reinterpret_cast<const float4 *>(kn + k4);
+      const float kv4[4] = {kk.x, kk.y, kk.z, kk.w};
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        s[k4 + u] = __fmul_rn(s[k4 + u], dc);
+        pk[k4 + u] = __fmul_rn(s[k4 + u], kv4[u]);
+      }
+    }
+    sums<false>(pk, pk, c, o, kv);
+    return kv;
+  }
+  template <bool MORE>
+  __device__ __forceinline__ void advance(const float *kn, const float *qn, const float *kn1, float value, float bt, float dc1, int c,
+                                          float &o, float &kv) {
+    const float delta = __fmul_rn(__fsub_rn(value, kv), bt);
+    float po[kRows], pk[kRows];
+#pragma unroll
+    for (int k4 = 0; k4 < kRows; k4 += 4) {
+      const float4 kk = *reinterpret_cast<const float4 *>(kn + k4);
+      const float4 qq = *reinterpret_cast<const float4 *>(qn + k4);
+      const float4 k1 = MORE ? *reinterpret_cast<const float4 *>(kn1 + k4) : kk;
+      const float kv4[4] = {kk.x, kk.y, kk.z, kk.w}, qv4[4] = {qq.x, qq.y, qq.z, qq.w}, kw4[4] = {k1.x, k1.y, k1.z, k1.w};
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        float &row = s[k4 + u];
+        row = __fadd_rn(row, __fmul_rn(kv4[u], delta));
+        po[k4 + u] = __fmul_rn(row, qv4[u]);
+        if (MORE) {
+          row = __fmul_rn(row, dc1);
+          pk[k4 + u] = __fmul_rn(row, kw4[u]);
+        }
+      }
+    }
+    if (MORE) {
+      sums<true>(po, pk, c, o, kv);
+    } else {
+      float unused;
+      sums<false>(po, po, c, unused, o);
+    }
+  }
+};
+
+// One lane's rows of its two columns (fast form).
+template <int DK> struct FastColumns {
+  static constexpr int kParts = 8, kRows = DK / kParts, kLanes = 32 / kParts;
+  Pair s[2][kRows / 2];
+
+  __device__ __forceinline__ void load(const float *col, int64_t dv) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int i = 0; i < kRows / 2; ++i)
+        s[j][i] = make_pair(col[2 * i * dv + j], col[(2 * i + 1) * dv + j]);
+  }
+  __device__ __forceinline__ void store(float *col, int64_t dv) const {
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int i = 0; i < kRows / 2; ++i) {
+        const float2 rows = unpack(s[j][i]);
+        col[2 * i * dv + j] = rows.x;
+        col[(2 * i + 1) * dv + j] = rows.y;
+      }
+  }
+  static __device__ __forceinline__ float halves(Pair p) {
+    const float2 v = unpack(p);
+    return v.x + v.y;
+  }
+  static __device__ __forceinline__ float over_parts(float x) {
+#pragma unroll
+    for (int o = kLanes; o < 32; o <<= 1)
+      x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+  }
+  __device__ __forceinline__ float2 first(const float *kn, float dc) {
+    Pair kv[2] = {make_pair(0.0f, 0.0f), make_pair(0.0f, 0.0f)};
+#pragma unroll
+    for (int i = 0; i < kRows / 2; i += 2) {
+      const Pair2 kk = *reinterpret_cast<const Pair2 *>(kn + 2 * i);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        s[j][i] = mul2(s[j][i], make_pair(dc, dc));
+        s[j][i + 1] = mul2(s[j][i + 1], make_pair(dc, dc));
+        kv[j] = fma2(s[j][i + 1], kk.y, fma2(s[j][i], kk.x, kv[j]));
+      }
+    }
+    return make_float2(over_parts(halves(kv[0])), over_parts(halves(kv[1])));
+  }
+  // o: of column 0 in the lanes of even parts, of column 1 in the others.
+  template <bool MORE>
+  __device__ __forceinline__ void advance(const float *kn, const float *qn, const float *kn1, float2 value, float bt, float dc1, bool odd,
+                                          float &o, float2 &kv) {
+    const float d0 = (value.x - kv.x) * bt, d1 = (value.y - kv.y) * bt;
+    const Pair delta[2] = {make_pair(d0, d0), make_pair(d1, d1)}, decay = make_pair(dc1, dc1);
+    Pair o2[2] = {make_pair(0.0f, 0.0f), make_pair(0.0f, 0.0f)}, kv2[2] = {o2[0], o2[0]};
+#pragma unroll
+    for (int i = 0; i < kRows / 2; i += 2) {
+      const Pair2 kk = *reinterpret_cast<const Pair2 *>(kn + 2 * i);
+      const Pair2 qq = *reinterpret_cast<const Pair2 *>(qn + 2 * i);
+      const Pair2 k1 = MORE ? *reinterpret_cast<const Pair2 *>(kn1 + 2 * i) : kk;
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          Pair &row = s[j][i + u];
+          row = fma2(u ? kk.y : kk.x, delta[j], row); // two rows as token t leaves them
+          o2[j] = fma2(row, u ? qq.y : qq.x, o2[j]);
+          if (MORE) {
+            row = mul2(row, decay); // decayed for token t + 1
+            kv2[j] = fma2(row, u ? k1.y : k1.x, kv2[j]);
+          }
+        }
+    }
+    if (MORE)
+      kv = make_float2(over_parts(halves(kv2[0])), over_parts(halves(kv2[1])));
+    const float o0 = halves(o2[0]), o1 = halves(o2[1]);
+    o = (odd ? o1 : o0) + __shfl_xor_sync(0xffffffffu, odd ? o0 : o1, kLanes);
+#pragma unroll
+    for (int x = 2 * kLanes; x < 32; x <<= 1)
+      o += __shfl_xor_sync(0xffffffffu, o, x);
+  }
+};
+
+template <int DK, bool EXACT>
 __global__ void __launch_bounds__(32 * kSplitWarps)
 gdn_recurrence_split_kernel(const uint16_t *__restrict__ conv, const float *__restrict__ qn,
                             const float *__restrict__ kn, const float *__restrict__ beta,
                             const float *__restrict__ decay, float *__restrict__ state, int S, int nk,
                             int nv, int dv, uint16_t *__restrict__ out) {
-  constexpr int kRows = DK / kSplitLanes; // state rows per lane
-  using Chunk = SplitChunk<DK>;
-  extern __shared__ __align__(16) unsigned char split_sm[]; // Chunk [kSplitWarps][3]
+  using Columns = std::conditional_t<EXACT, ExactColumn<DK>, FastColumns<DK>>;
+  constexpr int kParts = Columns::kParts, kRows = Columns::kRows, kLanes = Columns::kLanes, kLaneCols = kSplitCols / kLanes;
+  using Chunk = SplitChunk<DK, kParts>;
+  extern __shared__ __align__(16) unsigned char split_sm[]; // Chunk [3]
   grid_dependency_sync();
   const int h = blockIdx.x;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = lane % kSplitCols, part = lane / kSplitCols;
-  const int v0 = (blockIdx.y * kSplitWarps + warp) * kSplitCols, v = v0 + c;
-  if (v0 >= dv) // the column groups need not fill the last CTA
-    return;
-  Chunk *chunks = reinterpret_cast<Chunk *>(split_sm) + warp * 3;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, c = lane % kLanes, part = lane / kLanes;
+  const int cta_v0 = blockIdx.y * kSplitWarps * kSplitCols, at = warp * kSplitCols + c * kLaneCols, v = cta_v0 + at;
+  const bool active = v < dv; // the column groups need not fill the last CTA
+  Chunk *chunks = reinterpret_cast<Chunk *>(split_sm);
   const int kh = h / (nv / nk);
   const int64_t channels = 2 * static_cast<int64_t>(nk) * DK + static_cast<int64_t>(nv) * dv;
-  float *col = state + static_cast<int64_t>(h) * DK * dv + static_cast<int64_t>(part) * kRows * dv + v;
+  float *col = state + static_cast<int64_t>(h) * DK * dv + static_cast<int64_t>(part) * kRows * dv + (active ? v : 0);
 
-  float s[kRows];
-#pragma unroll
-  for (int k = 0; k < kRows; ++k)
-    s[k] = col[static_cast<int64_t>(k) * dv];
+  Columns columns;
+  columns.load(col, dv); // an idle warp walks along with the first columns and stores nothing
 
   auto copy = [](void *dst, const void *src, auto bytes) {
     if (decltype(bytes)::value == 16)
@@ -465,11 +647,12 @@ gdn_recurrence_split_kernel(const uint16_t *__restrict__ conv, const float *__re
                    "n"(decltype(bytes)::value)
                    : "memory");
   };
-  // Requests chunk `index` (tokens 8 index .. 8 index + 7, those below S) and closes the copy group.
+  // Requests chunk `index` (tokens 8 index .. 8 index + 7, those below S).
   auto request = [&](int index) {
     Chunk &ch = chunks[index % 3];
     const int t0 = index * kSplitChunk;
-    for (int i = lane; i < kSplitChunk * (2 * DK / 4); i += 32) { // 16-byte pieces of k and q
+#pragma unroll
+    for (int i = tid; i < kSplitChunk * (2 * DK / 4); i += 32 * kSplitWarps) { // 16-byte pieces of k and q
       const int token = i / (2 * DK / 4), piece = i % (2 * DK / 4);
       if (t0 + token < S) {
         const int which = piece / (DK / 4), row = (piece % (DK / 4)) * 4;
@@ -477,103 +660,74 @@ gdn_recurrence_split_kernel(const uint16_t *__restrict__ conv, const float *__re
         copy(&ch.kq[token][which][row / kRows][row % kRows], src, std::integral_constant<int, 16>());
       }
     }
-    if (lane < kSplitChunk && t0 + lane < S) {
-      copy(&ch.value[lane][0], conv + (t0 + lane) * channels + 2 * static_cast<int64_t>(nk) * DK + h * dv + v0,
+    const int token = tid / kSplitWarps, piece = tid % kSplitWarps; // 8 values each
+    if (token < kSplitChunk && t0 + token < S && cta_v0 + piece * kSplitCols < dv)
+      copy(&ch.value[token][piece * kSplitCols],
+           conv + (t0 + token) * channels + 2 * static_cast<int64_t>(nk) * DK + h * dv + cta_v0 + piece * kSplitCols,
            std::integral_constant<int, 2 * kSplitCols>());
-      copy(&ch.dc[lane], decay + static_cast<int64_t>(t0 + lane) * nv + h, std::integral_constant<int, 4>());
-      copy(&ch.bt[lane], beta + static_cast<int64_t>(t0 + lane) * nv + h, std::integral_constant<int, 4>());
+    if (tid >= 64 && tid < 64 + kSplitChunk && t0 + tid - 64 < S) {
+      copy(&ch.dc[tid - 64], decay + static_cast<int64_t>(t0 + tid - 64) * nv + h, std::integral_constant<int, 4>());
+      copy(&ch.bt[tid - 64], beta + static_cast<int64_t>(t0 + tid - 64) * nv + h, std::integral_constant<int, 4>());
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  auto over_parts = [](float x) { // the lanes of a column hold its row groups' partial sums
-#pragma unroll
-    for (int o = kSplitCols; o < 32; o <<= 1)
-      x += __shfl_xor_sync(0xffffffffu, x, o);
-    return x;
-  };
   uint16_t *out_col = out + static_cast<int64_t>(h) * dv + v;
   const int64_t out_stride = static_cast<int64_t>(nv) * dv;
+  using Values = std::conditional_t<EXACT, float, float2>; // per column of this lane
+  auto values = [&](const Chunk *ch, int slot) {
+    if constexpr (EXACT)
+      return bf16_to_f32(ch->value[slot][at]);
+    else
+      return make_float2(bf16_to_f32(ch->value[slot][at]), bf16_to_f32(ch->value[slot][at + 1]));
+  };
 
   request(0);
   request(1);
-  float kv = 0.0f, bt = 0.0f, value = 0.0f;
+  Values kv{}, value{};
+  float bt = 0.0f, o = 0.0f;
   int slot = 0, cur_index = 0; // token t is slot `slot` of chunk `cur_index` (buffer cur_index % 3)
   const Chunk *cur = chunks;
   for (int t = 0; t < S; ++t) {
-    if (slot == 0) { // chunk index + 2 goes into the buffer of the chunk that has just been left
-      __syncwarp();
+    if (slot == 0) { // this chunk and the next have landed; chunk index + 2 goes where everyone has just left
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();
       request(cur_index + 2);
-      asm volatile("cp.async.wait_group 1;" ::: "memory"); // all but the newest group: this chunk and the next
-      __syncwarp();
     }
-    if (t == 0) { // the first token's decay and first chain on their own
-      const float dc = cur->dc[0];
+    if (t == 0) {
       bt = cur->bt[0];
-      value = bf16_to_f32(cur->value[0][c]);
-#pragma unroll
-      for (int k4 = 0; k4 < kRows; k4 += 4) {
-        const float4 kk = *reinterpret_cast<const float4 *>(&cur->kq[0][0][part][k4]);
-        const float kv4[4] = {kk.x, kk.y, kk.z, kk.w};
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          s[k4 + u] *= dc;
-          kv = __fmaf_rn(s[k4 + u], kv4[u], kv);
-        }
-      }
-      kv = over_parts(kv);
+      value = values(cur, 0);
+      if constexpr (EXACT)
+        kv = columns.first(cur->kq[0][0][part], cur->dc[0], c);
+      else
+        kv = columns.first(cur->kq[0][0][part], cur->dc[0]);
     }
-    const float delta = (value - kv) * bt;
-    float o = 0.0f;
     // where token t + 1 lives
     const int nslot = slot + 1 == kSplitChunk ? 0 : slot + 1;
     const int nindex = nslot == 0 ? cur_index + 1 : cur_index;
     const Chunk *nxt = nslot == 0 ? chunks + nindex % 3 : cur;
+    const float *k0 = cur->kq[slot][0][part], *q0 = cur->kq[slot][1][part], *k1 = nxt->kq[nslot][0][part];
     if (t + 1 < S) {
-      const float dc1 = nxt->dc[nslot];
-      bt = nxt->bt[nslot];
-      value = bf16_to_f32(nxt->value[nslot][c]);
-      float kv1[2] = {0.0f, 0.0f}, o2[2] = {0.0f, 0.0f}; // two interleaved partial sums per chain
-#pragma unroll
-      for (int k4 = 0; k4 < kRows; k4 += 4) {
-        const float4 kk = *reinterpret_cast<const float4 *>(&cur->kq[slot][0][part][k4]);
-        const float4 qq = *reinterpret_cast<const float4 *>(&cur->kq[slot][1][part][k4]);
-        const float4 kn1 = *reinterpret_cast<const float4 *>(&nxt->kq[nslot][0][part][k4]);
-        const float kv4[4] = {kk.x, kk.y, kk.z, kk.w};
-        const float qv4[4] = {qq.x, qq.y, qq.z, qq.w};
-        const float kw4[4] = {kn1.x, kn1.y, kn1.z, kn1.w};
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          s[k4 + u] = __fmaf_rn(kv4[u], delta, s[k4 + u]); // row k as token t leaves it
-          o2[u & 1] = __fmaf_rn(s[k4 + u], qv4[u], o2[u & 1]);
-          s[k4 + u] *= dc1;                                // decayed for token t + 1
-          kv1[u & 1] = __fmaf_rn(s[k4 + u], kw4[u], kv1[u & 1]);
-        }
-      }
-      o = o2[0] + o2[1];
-      kv = over_parts(kv1[0] + kv1[1]);
+      const float bt1 = nxt->bt[nslot], dc1 = nxt->dc[nslot];
+      const Values value1 = values(nxt, nslot);
+      if constexpr (EXACT)
+        columns.template advance<true>(k0, q0, k1, value, bt, dc1, c, o, kv);
+      else
+        columns.template advance<true>(k0, q0, k1, value, bt, dc1, part & 1, o, kv);
+      bt = bt1;
+      value = value1;
     } else {
-#pragma unroll
-      for (int k4 = 0; k4 < kRows; k4 += 4) {
-        const float4 kk = *reinterpret_cast<const float4 *>(&cur->kq[slot][0][part][k4]);
-        const float4 qq = *reinterpret_cast<const float4 *>(&cur->kq[slot][1][part][k4]);
-        const float kv4[4] = {kk.x, kk.y, kk.z, kk.w};
-        const float qv4[4] = {qq.x, qq.y, qq.z, qq.w};
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          s[k4 + u] = __fmaf_rn(kv4[u], delta, s[k4 + u]);
-          o = __fmaf_rn(s[k4 + u], qv4[u], o);
-        }
-      }
+      if constexpr (EXACT)
+        columns.template advance<false>(k0, q0, k0, value, bt, 1.0f, c, o, kv);
+      else
+        columns.template advance<false>(k0, q0, k0, value, bt, 1.0f, part & 1, o, kv);
     }
-    o = over_parts(o);
-    if (part == 0)
-      out_col[t * out_stride] = f32_to_bf16(o);
+    if (active && part < kLaneCols)
+      out_col[t * out_stride + part] = f32_to_bf16(o);
     slot = nslot, cur_index = nindex, cur = nxt;
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-#pragma unroll
-  for (int k = 0; k < kRows; ++k)
-    col[static_cast<int64_t>(k) * dv] = s[k];
+  if (active)
+    columns.store(col, dv);
 }
 
 size_t gdn_scratch_floats(int64_t S, int nk, int nv, int dk) {
@@ -604,14 +758,17 @@ cudaError_t launch_gated_delta_net(const uint16_t *conv, const uint16_t *a, cons
     const char *flag = std::getenv("LLMCP_B200_GDN_PIPELINE");
     return !(flag && flag[0] == '0');
   }();
-  if (dk == 128 && S > 1 && fast && dv % kSplitCols == 0 && S < (1 << 30)) {
-    constexpr size_t split_bytes = kSplitWarps * 3 * sizeof(SplitChunk<128>);
-    if (cudaError_t e = opt_in_shared_memory(reinterpret_cast<const void *>(gdn_recurrence_split_kernel<128>), split_bytes);
-        e != cudaSuccess)
-      return e;
+  // Copies of 16 bytes: whole groups of eight value columns, on 16-byte boundaries.
+  const bool split = dk == 128 && S > 1 && S < (1 << 30) && dv % kSplitCols == 0 && reinterpret_cast<uintptr_t>(conv) % 16 == 0 &&
+                     reinterpret_cast<uintptr_t>(scratch) % 16 == 0;
+  if (split && (fast || pipelined)) {
+    const auto kernel = fast ? gdn_recurrence_split_kernel<128, false> : gdn_recurrence_split_kernel<128, true>;
+    constexpr size_t fast_bytes = 3 * sizeof(SplitChunk<128, FastColumns<128>::kParts>), exact_bytes = 3 * sizeof(SplitChunk<128, ExactColumn<128>::kParts>);
+    static_assert(fast_bytes <= 48 * 1024 && exact_bytes <= 48 * 1024, "no opt-in needed");
+    const size_t split_bytes = fast ? fast_bytes : exact_bytes;
     const int groups = dv / kSplitCols;
-    launch_chained(gdn_recurrence_split_kernel<128>, dim3(nv, (groups + kSplitWarps - 1) / kSplitWarps), dim3(32 * kSplitWarps),
-                   split_bytes, stream, conv, qn, kn, beta, decay, state, static_cast<int>(S), nk, nv, dv, out);
+    launch_chained(kernel, dim3(nv, (groups + kSplitWarps - 1) / kSplitWarps), dim3(32 * kSplitWarps), split_bytes, stream, conv, qn, kn,
+                   beta, decay, state, static_cast<int>(S), nk, nv, dv, out);
   }
   else if (dk == 128 && S > 1 && pipelined)
     launch_chained(gdn_recurrence_pipelined_kernel<128>, dim3(grid), dim3(32), 0, stream, conv, qn, kn, beta, decay, state, S, nk, nv, dv, out);

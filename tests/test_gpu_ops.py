@@ -571,3 +571,29 @@ def test_gemm_tma_tile_widths(monkeypatch, tile, M, N, K):
         torch.cuda.synchronize()
         assert int(status.item()) == 0
         assert np.array_equal(y.cpu().numpy().view(np.uint32), want.view(np.uint32)), form
+
+
+@pytest.mark.parametrize("fast", [False, True])
+@pytest.mark.parametrize("S,nk,nv,dv", [(2, 2, 8, 128), (7, 1, 1, 8), (8, 2, 4, 40), (9, 2, 2, 128), (16, 1, 2, 64), (17, 2, 4, 32),
+                                        (25, 4, 8, 136)])
+def test_gated_delta_net_chunk_edges(fast, S, nk, nv, dv):
+    """The many-token recurrence at the edges of its 8-token chunks and 32-column CTAs: exact mode bit for bit, fast mode
+    within f32 rounding of the state (sums of 128 products, S times) and two bf16 steps of the largest output."""
+    dk = 128
+    rng = np.random.default_rng(S + nv + dv)
+    channels = 2 * nk * dk + nv * dv
+    conv, a, b = rand_bf16(rng, S, channels), rand_bf16(rng, S, nv), rand_bf16(rng, S, nv)
+    a_log = (rng.standard_normal(nv) * 0.2).astype(np.float32)
+    dt, state = rand_bf16(rng, nv, scale=0.2), (rng.standard_normal((nv, dk, dv)) * 0.1).astype(np.float32)
+    want, want_state = oracle.gated_delta_net(conv, a, b, a_log, dt, state, nk, nv, dk, dv)
+    L.set_mode("fast" if fast else "exact")
+    try:
+        got, got_state = L.ops.gated_delta_net(conv, a, b, a_log, dt, state, nk, nv, dk, dv)
+    finally:
+        L.set_mode("exact")
+    if fast:
+        assert np.abs(f(got) - f(want)).max() <= 2.0 ** -7 * np.abs(f(want)).max()
+        assert np.abs(got_state - want_state).max() <= 1e-4 * np.abs(want_state).max()
+    else:
+        assert np.array_equal(got, want)
+        assert np.array_equal(got_state.view(np.uint32), want_state.view(np.uint32))

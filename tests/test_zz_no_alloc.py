@@ -70,6 +70,21 @@ def test_noalloc_matches_allocating_entry_point_twice():
         assert np.array_equal(state.view(np.uint32), oracle_state.view(np.uint32))
 
 
+def test_noalloc_takes_inputs_off_the_16_byte_boundary():
+    """Values two bytes off a 16-byte boundary go through the kernel without 16-byte copies: the same bits."""
+    torch = pytest.importorskip("torch")
+    S, nk, nv, dk, dv = 9, 2, 4, 128, 128
+    x = _inputs(np.random.default_rng(5), S, nk, nv, dk, dv)
+    _, want, want_state = _noalloc(torch, x, S, nk, nv, dk, dv)
+    dev, out = _upload(torch, x, S, nv, dv)
+    shifted = torch.empty(dev["conv"].numel() + 1, dtype=torch.int16, device="cuda")
+    shifted[1:] = dev["conv"].reshape(-1)
+    dev["conv"] = shifted[1:]
+    assert _call(torch, dev, out, S, nk, nv, dk, dv) == 0, L.last_error()
+    assert np.array_equal(out.cpu().numpy().view(np.uint16), want)
+    assert np.array_equal(dev["state"].cpu().numpy().view(np.uint32), want_state.view(np.uint32))
+
+
 def test_noalloc_leaves_free_device_memory_unchanged():
     """After one call per kernel (one token, several tokens) further calls take no device memory: the
     free byte count of the GPU is the same before and after them (inputs and output are uploaded
