@@ -745,7 +745,15 @@ static void run_linears(const F16Planes &planes, const int8_t *aq, const float *
   }
   const bool tma = gemm_error && planes.form >= 0 && planes.ast && jobs[0].w->d32t;
   const bool f16 = tma && planes.form >= kGemmF16;
-  if (tma) { // the shared input once: scales block-major, and for the f16 forms the int8 values as f16
+  // Matrices that the narrow-tile GEMM takes read the scales as they are; for the others the shared input is laid out
+  // once: scales block-major, and for the f16 forms the int8 values as f16.
+  bool few[kMaxGemvJobs], planes_needed = false;
+  for (int i = 0; i < count; ++i) {
+    few[i] = tma && planes.form == kGemmI8Packed && gemm_few_preferred(static_cast<int>(S), jobs[i].w->N) &&
+             gemm_few_takes_row_scales(static_cast<int>(S), jobs[i].w->K, as);
+    planes_needed = planes_needed || !few[i];
+  }
+  if (tma && planes_needed) {
     if (f16)
       launch_act_to_f16(aq, as, S, jobs[0].w->K, planes.ah, planes.ast, stream);
     else
@@ -766,7 +774,9 @@ static void run_linears(const F16Planes &planes, const int8_t *aq, const float *
         throw std::runtime_error("gemm: cudaStreamWaitEvent");
     }
     cudaError_t e =
-        tma ? launch_gemm_q8_tma(planes.form, f16 ? planes.ah : static_cast<const void *>(aq), planes.ast, static_cast<int>(S),
+        few[i] ? launch_gemm_q8_few(aq, as, true, static_cast<int>(S), jobs[i].w->K, jobs[i].w->q, jobs[i].w->d32t, jobs[i].w->N,
+                                    jobs[i].y, jobs[i].y_dtype, jobs[i].activation, nullptr, gemm_error, stream_i)
+        : tma ? launch_gemm_q8_tma(planes.form, f16 ? planes.ah : static_cast<const void *>(aq), planes.ast, static_cast<int>(S),
                                  jobs[i].w->K, f16 ? jobs[i].w->h : static_cast<const void *>(jobs[i].w->q), jobs[i].w->d32t,
                                  jobs[i].w->N, jobs[i].y, jobs[i].y_dtype, jobs[i].activation, nullptr, gemm_error, stream_i)
         : gemm_error ? launch_gemm_q8_tc(aq, as, static_cast<int>(S), jobs[i].w->K, jobs[i].w->q, jobs[i].w->d32,

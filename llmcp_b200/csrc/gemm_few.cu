@@ -70,7 +70,10 @@ __device__ __forceinline__ void fold2(float &c0, float &c1, int d0, int d1, floa
 }
 
 // fault (test hook): 1 = the producer announces the first stage's bytes but never issues its copies.
-template <int WN, int WM, int NT, int KS, int STAGES, bool DOTS>
+__device__ __forceinline__ float component(float4 v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
+
+// ROWS: the activations' scales come as they are quantised, [M][K/32]; otherwise block-major.
+template <int WN, int WM, int NT, int KS, int STAGES, bool DOTS, bool ROWS>
 __global__ void __launch_bounds__(Few<WN, WM, NT, KS, STAGES>::kThreads, 2)
 gemm_q8_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
                    const __grid_constant__ CUtensorMap map_ws, const __grid_constant__ CUtensorMap map_as, int M, int K, int N,
@@ -116,7 +119,7 @@ gemm_q8_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
           }
           uint8_t *scales = stage + F::kBoxes * (F::kBoxW + F::kBoxA);
           tma_load_2d(scales, &map_ws, n0, it * F::kBlocks, &bars.full[s]);
-          tma_load_2d(scales + F::kScalesW, &map_as, m0, it * F::kBlocks, &bars.full[s]);
+          tma_load_2d(scales + F::kScalesW, &map_as, ROWS ? it * F::kBlocks : m0, ROWS ? m0 : it * F::kBlocks, &bars.full[s]);
         }
       }
       // Leaving after a failed wait: copies already requested still write into this CTA's shared memory.
@@ -149,9 +152,19 @@ gemm_q8_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const uint8_t *w_rows = stage + wn * 16 * 128, *a_rows = stage + F::kBoxes * F::kBoxW + wm * 8 * NT * 128;
         const float *w_scale = reinterpret_cast<const float *>(stage + F::kBoxes * (F::kBoxW + F::kBoxA)) + wn * 16 + row8;
         // column 2t of the result is activation row 2t of the fragment's order, column 2t + 1 row 2t + 1
-        const float *a_scale = reinterpret_cast<const float *>(stage + F::kBoxes * (F::kBoxW + F::kBoxA) + F::kScalesW) + wm * 8 * NT;
+        const float *a_scale = reinterpret_cast<const float *>(stage + F::kBoxes * (F::kBoxW + F::kBoxA) + F::kScalesW) + wm * 8 * NT * (ROWS ? F::kBlocks : 1);
         const int c0 = t < 2 ? 4 * t : 4 * t - 7, c1 = c0 + 2;
+        // The scales as they are quantised: four blocks of a row at a time where the registers allow it.
+        constexpr bool kFour = ROWS && NT <= 2;
+        float4 four[kFour ? NT : 1][2];
         auto fold = [&](int b) {
+          if (kFour && b % 4 == 0) {
+#pragma unroll
+            for (int j = 0; j < (kFour ? NT : 0); ++j) {
+              four[j][0] = *reinterpret_cast<const float4 *>(a_scale + (j * 8 + c0) * F::kBlocks + b);
+              four[j][1] = *reinterpret_cast<const float4 *>(a_scale + (j * 8 + c1) * F::kBlocks + b);
+            }
+          }
           const uint8_t *w_box = w_rows + (b / 4) * F::kBoxW + offset[b % 4], *a_box = a_rows + (b / 4) * F::kBoxA + offset[b % 4];
           const uint2 lo = *reinterpret_cast<const uint2 *>(w_box);
           const uint2 hi = *reinterpret_cast<const uint2 *>(w_box + 8 * 128);
@@ -159,7 +172,13 @@ gemm_q8_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
           for (int j = 0; j < NT; ++j) {
             const uint2 x = *reinterpret_cast<const uint2 *>(a_box + j * 8 * 128);
-            const float2 sa = make_float2(a_scale[b * F::kRowsA + j * 8 + c0], a_scale[b * F::kRowsA + j * 8 + c1]);
+            float2 sa;
+            if (kFour)
+              sa = make_float2(component(four[j % (kFour ? NT : 1)][0], b % 4), component(four[j % (kFour ? NT : 1)][1], b % 4));
+            else if (ROWS)
+              sa = make_float2(a_scale[(j * 8 + c0) * F::kBlocks + b], a_scale[(j * 8 + c1) * F::kBlocks + b]);
+            else
+              sa = make_float2(a_scale[b * F::kRowsA + j * 8 + c0], a_scale[b * F::kRowsA + j * 8 + c1]);
             int d[4];
             block_dots(d, lo, hi, x);
             fold2(acc[j][0], acc[j][1], d[0], d[1], sa, w0);
@@ -209,7 +228,8 @@ gemm_q8_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 
 struct FewCall {
   const int8_t *aq;
-  const float *ast;
+  const float *as; // [M][K/32], or block-major
+  bool rows;
   int M, K;
   const int8_t *wq;
   const float *wst;
@@ -223,15 +243,18 @@ struct FewCall {
   int fault, sm_count;
 };
 
-template <int WN, int WM, int NT, int KS, int STAGES> cudaError_t launch_few(const FewCall &c) {
+template <int WN, int WM, int NT, int KS, int STAGES, bool MAY_BE_ROWS> cudaError_t launch_few(const FewCall &c) {
   using F = Few<WN, WM, NT, KS, STAGES>;
   const int nb = c.K / kBlock;
   CUtensorMap map_w, map_a, map_ws, map_as;
   if (!gemm_operand_map(&map_w, c.wq, c.N, c.K, false, F::kRowsW) || !gemm_operand_map(&map_a, c.aq, c.M, c.K, false, F::kRowsA) ||
       !gemm_scale_map(&map_ws, c.wst, c.N, c.N, nb, F::kBlocks, F::kRowsW) ||
-      !gemm_scale_map(&map_as, c.ast, c.M, gemm_tc16_scale_pitch(c.M), nb, F::kBlocks, F::kRowsA))
+      !(c.rows ? gemm_scale_map(&map_as, c.as, nb, nb, c.M, F::kRowsA, F::kBlocks)
+               : gemm_scale_map(&map_as, c.as, c.M, gemm_tc16_scale_pitch(c.M), nb, F::kBlocks, F::kRowsA)))
     return cudaErrorNotSupported;
-  auto kernel = c.dots_out ? gemm_q8_few_kernel<WN, WM, NT, KS, STAGES, true> : gemm_q8_few_kernel<WN, WM, NT, KS, STAGES, false>;
+  auto kernel = c.dots_out ? gemm_q8_few_kernel<WN, WM, NT, KS, STAGES, true, false>
+                : c.rows   ? gemm_q8_few_kernel<WN, WM, NT, KS, STAGES, false, MAY_BE_ROWS>
+                           : gemm_q8_few_kernel<WN, WM, NT, KS, STAGES, false, false>;
   if (cudaError_t e = opt_in_shared_memory(reinterpret_cast<const void *>(kernel), F::kSmemBytes); e != cudaSuccess)
     return e;
   const int m_tiles = (c.M + F::kRowsA - 1) / F::kRowsA, tiles = m_tiles * ((c.N + F::kRowsW - 1) / F::kRowsW);
@@ -246,15 +269,30 @@ template <int WN, int WM, int NT, int KS, int STAGES> cudaError_t launch_few(con
 // rows always (248320 weight rows: 246 us against 460); up to 64 rows until an SM has more than four tiles (9216 weight
 // rows 26 us against 36; 248320: 563 against 460); beyond that while two of three SMs at most have one (128 x 2560 x 9216
 // 64 us against 72, 128 x 4096 x 2560 26 against 24).
-bool gemm_few_preferred(int M, int N, int sm_count) {
+bool gemm_few_preferred(int M, int N) {
+  if (gemm_forced_tile())
+    return false;
+  int sms = 148;
+  if (current_sm_count(&sms) != cudaSuccess || sms <= 0)
+    sms = 148;
   const int64_t tiles = static_cast<int64_t>((M + 63) / 64) * ((N + 63) / 64);
-  return M <= 32 || (M <= 64 ? tiles <= 4 * sm_count : 3 * tiles <= 2 * sm_count);
+  return M <= 32 || (M <= 64 ? tiles <= 4 * sms : 3 * tiles <= 2 * sms);
 }
 
-cudaError_t launch_gemm_q8_few(const int8_t *aq, const float *ast, int M, int K, const int8_t *wq, const float *wst, int N,
-                               void *y, int y_dtype, int activation, int32_t *dots_out, int *error_flag, cudaStream_t stream,
+// More than 32 rows: a launch less in front of every GEMM (64 sequences decoded together, 13 steps: 105 -> 98 ms).  Up to 32
+// rows their copies of 32 bytes per row cost more than that launch (a 23-token prompt: 4.8 ms block-major, 5.0 so).
+bool gemm_few_takes_row_scales(int M, int K, const float *as) {
+  return M > 32 && K % 128 == 0 && reinterpret_cast<uintptr_t>(as) % 16 == 0;
+}
+
+cudaError_t launch_gemm_q8_few(const int8_t *aq, const float *as, bool row_scales, int M, int K, const int8_t *wq, const float *wst,
+                               int N, void *y, int y_dtype, int activation, int32_t *dots_out, int *error_flag, cudaStream_t stream,
                                uint32_t spin_limit, int fault) {
-  FewCall call = {aq, ast, M, K, wq, wst, N, y, y_dtype, activation, dots_out, error_flag, stream, spin_limit, fault, 148};
+  if (M <= 0 || N % 8 != 0 || K % kBlock != 0 || (row_scales && (dots_out || !gemm_few_takes_row_scales(M, K, as))))
+    return cudaErrorInvalidValue;
+  if (spin_limit == 0)
+    spin_limit = kSpinLimit;
+  FewCall call = {aq, as, row_scales, M, K, wq, wst, N, y, y_dtype, activation, dots_out, error_flag, stream, spin_limit, fault, 148};
   int sms = 0;
   if (current_sm_count(&sms) == cudaSuccess && sms > 0)
     call.sm_count = sms;
@@ -263,10 +301,10 @@ cudaError_t launch_gemm_q8_few(const int8_t *aq, const float *ast, int M, int K,
   // The widest tile that still gives four of five SMs a CTA.
   const int64_t enough = call.sm_count * 4 / 5;
   if (rows * ((N + 63) / 64) >= enough)
-    return narrow ? launch_few<4, 2, 2, 128, 7>(call) : launch_few<4, 2, 4, 128, 6>(call);
+    return narrow ? launch_few<4, 2, 2, 128, 7, false>(call) : launch_few<4, 2, 4, 128, 6, true>(call);
   if (rows * ((N + 31) / 32) >= enough)
-    return narrow ? launch_few<2, 2, 2, 256, 6>(call) : launch_few<2, 4, 2, 256, 4>(call);
-  return narrow ? launch_few<1, 4, 1, 256, 7>(call) : launch_few<1, 4, 2, 256, 4>(call);
+    return narrow ? launch_few<2, 2, 2, 256, 6, false>(call) : launch_few<2, 4, 2, 256, 4, true>(call);
+  return narrow ? launch_few<1, 4, 1, 256, 7, false>(call) : launch_few<1, 4, 2, 256, 4, true>(call);
 }
 
 } // namespace llmcp_b200

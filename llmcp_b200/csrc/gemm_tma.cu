@@ -461,18 +461,11 @@ template <bool F16, int TN> cudaError_t launch_tile(const GemmCall &c) {
   return cudaGetLastError();
 }
 
-// LLMCP_B200_GEMM_TILE=64|96|128: the tile width for every shape, few rows included; 0 = not set.
-int forced_tile() {
-  const char *flag = std::getenv("LLMCP_B200_GEMM_TILE");
-  const int forced = flag ? std::atoi(flag) : 0;
-  return forced == 64 || forced == 96 || forced == 128 ? forced : 0;
-}
-
 // Tile width for an M x N output: a CTA works through ceil(tiles / SMs) tiles, each at a cost that grows with its
 // width and has a part that does not (the hand-off of a block, worth about 72 columns: 23.4, 27.8 and
 // 33.7 us for one tile of K = 2560).
 int choose_tile(int M, int N, int sm_count) {
-  if (const int forced = forced_tile())
+  if (const int forced = gemm_forced_tile())
     return forced;
   const int64_t rows = (M + kTileM - 1) / kTileM;
   int best = 128;
@@ -496,19 +489,35 @@ template <bool F16> cudaError_t launch_form(const GemmCall &c) {
   }
 }
 
-// [rows][K/32] scales -> block-major f32 [K/32][ld]; scales are f32 (activations) or f16 bits (weights).
-__global__ void scales_block_major_kernel(const void *__restrict__ scales, int scales_are_f16, int64_t rows, int nb, int64_t ld,
-                                          float *__restrict__ out) {
+// [rows][K/32] scales -> block-major f32 [K/32][ld]; scales are f32 (activations) or f16 bits (weights).  A CTA turns
+// 32 x 32 scales through shared memory, so that reads and writes are both of whole lines (an element per thread wrote
+// with a stride of a plane's row).
+__global__ void __launch_bounds__(256)
+scales_block_major_kernel(const void *__restrict__ scales, int scales_are_f16, int64_t rows, int nb, int64_t ld, float *__restrict__ out) {
+  __shared__ float tile[32][33];
   grid_dependency_sync();
-  const int64_t total = rows * nb;
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total; i += stride) {
-    const int64_t r = i / nb, b = i % nb;
-    out[b * ld + r] = scales_are_f16 ? f16_bits_to_f32(static_cast<const uint16_t *>(scales)[i]) : static_cast<const float *>(scales)[i];
-  }
+  const int64_t r0 = blockIdx.x * static_cast<int64_t>(32);
+  const int b0 = blockIdx.y * 32, x = threadIdx.x & 31, y0 = threadIdx.x >> 5;
+#pragma unroll
+  for (int y = y0; y < 32; y += 8)
+    if (r0 + y < rows && b0 + x < nb) {
+      const int64_t i = (r0 + y) * nb + b0 + x;
+      tile[y][x] = scales_are_f16 ? f16_bits_to_f32(static_cast<const uint16_t *>(scales)[i]) : static_cast<const float *>(scales)[i];
+    }
+  __syncthreads();
+#pragma unroll
+  for (int y = y0; y < 32; y += 8)
+    if (r0 + x < rows && b0 + y < nb)
+      out[static_cast<int64_t>(b0 + y) * ld + r0 + x] = tile[x][y];
 }
 
 } // namespace
+
+int gemm_forced_tile() {
+  const char *flag = std::getenv("LLMCP_B200_GEMM_TILE");
+  const int forced = flag ? std::atoi(flag) : 0;
+  return forced == 64 || forced == 96 || forced == 128 ? forced : 0;
+}
 
 int64_t gemm_tc16_scale_pitch(int64_t M) { return (M + 3) / 4 * 4; }
 
@@ -528,8 +537,8 @@ void launch_weights_to_f16(const int8_t *wq, const uint16_t *wd, int64_t N, int 
 void launch_scales_block_major(const void *scales, int scales_are_f16, int64_t rows, int K, int64_t ld, float *out,
                                cudaStream_t stream) {
   const int nb = K / kBlock;
-  const int blocks = static_cast<int>(std::min<int64_t>((rows * nb + 255) / 256, 148 * 8));
-  launch_chained(scales_block_major_kernel, dim3(blocks), dim3(256), 0, stream, scales, scales_are_f16, rows, nb, ld, out);
+  launch_chained(scales_block_major_kernel, dim3(static_cast<unsigned>((rows + 31) / 32), (nb + 31) / 32), dim3(256), 0, stream, scales,
+                 scales_are_f16, rows, nb, ld, out);
 }
 
 cudaError_t launch_gemm_q8_tma(int form, const void *a, const float *ast, int M, int K, const void *w, const float *wst, int N,
@@ -550,8 +559,8 @@ cudaError_t launch_gemm_q8_tma(int form, const void *a, const float *ast, int M,
   case kGemmI8:
     return launch_form<false>(call);
   case kGemmI8Packed:
-    if (!forced_tile() && gemm_few_preferred(M, N, call.sm_count))
-      return launch_gemm_q8_few(static_cast<const int8_t *>(a), ast, M, K, static_cast<const int8_t *>(w), wst, N, y, y_dtype,
+    if (gemm_few_preferred(M, N))
+      return launch_gemm_q8_few(static_cast<const int8_t *>(a), ast, false, M, K, static_cast<const int8_t *>(w), wst, N, y, y_dtype,
                                 activation, dots_out, error_flag, stream, spin_limit, fault);
     return launch_form<false>(call);
   default:

@@ -102,10 +102,13 @@ cudaError_t launch_gemm_q8_tma(int form, const void *a, const float *ast, int M,
                                uint32_t spin_limit = 0, int fault = 0);
 // The same contraction in narrow tiles (gemm_few.cu); operands as for kGemmI8Packed, which takes this form by itself
 // where gemm_few_preferred.
-bool gemm_few_preferred(int M, int N, int sm_count);
-cudaError_t launch_gemm_q8_few(const int8_t *aq, const float *ast, int M, int K, const int8_t *wq, const float *wst, int N,
-                               void *y, int y_dtype, int activation, int32_t *dots_out, int *error_flag, cudaStream_t stream,
-                               uint32_t spin_limit, int fault);
+bool gemm_few_preferred(int M, int N);
+int gemm_forced_tile(); // LLMCP_B200_GEMM_TILE: the wide form's tile width, for every shape; 0 = not set
+// row_scales: `as` is [M][K/32] as the quantising kernels write it (where gemm_few_takes_row_scales), not block-major.
+bool gemm_few_takes_row_scales(int M, int K, const float *as);
+cudaError_t launch_gemm_q8_few(const int8_t *aq, const float *as, bool row_scales, int M, int K, const int8_t *wq, const float *wst,
+                               int N, void *y, int y_dtype, int activation, int32_t *dots_out, int *error_flag, cudaStream_t stream,
+                               uint32_t spin_limit = 0, int fault = 0);
 // status (device int, optional): bit 1 is raised when a token id lies outside [0, vocab); such a
 // row is written as zeros and the table is not read.
 // Second form of the tensor-core GEMM (gemm_tma.cu): the int8 operands held as f16 values and the
