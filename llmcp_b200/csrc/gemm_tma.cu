@@ -25,7 +25,8 @@
 // 87 -> 84, 1024 x 32 x 2560 42 -> 22.  Fragment-shaped tensor-memory loads (16x256b: fewer scale registers) read
 // tensor memory at a quarter of the rate and measured 160 us.
 //
-// One CTA per SM takes 128 x TN output tiles in turn, 576 threads:
+// One CTA per SM (two of 320 threads for TN = 64, out of step with each other) takes 128 x TN output tiles in turn,
+// 576 threads:
 //   warp  0     one lane issues the TMA loads (cp.async.bulk.tensor, 128-byte swizzle, no
 //               multicast): per stage a box of 128 (TN) rows x 128 bytes of K of each operand (four
 //               int8 or two f16 quantisation blocks) and those blocks' f32 scales of the tile's rows
@@ -33,7 +34,7 @@
 //               floats per block);
 //   warp  1     one lane issues the MMAs, two blocks into a tensor-memory slot (f16: two K = 16
 //               instructions per block, the first overwrites, the second accumulates), and commits the slot;
-//   warps 2-17  epilogue: tcgen05.ld a block (thread = row, TN / 4 columns), hand the slot back after its last
+//   warps 2-17  epilogue (2-9 for TN = 64): tcgen05.ld a block (thread = row, 24 or 32 columns), hand the slot back after its last
 //               block's load, then the arithmetic with the scales read from shared memory.
 // Hand-offs are mbarriers; every wait is bounded (spin_limit polls) and a timed-out wait raises an
 // abort flag that all roles observe, so a protocol error ends the kernel with an error code instead
@@ -56,8 +57,6 @@ using namespace tc;
 
 constexpr int kTileM = 128;
 constexpr int kEpilogueWarp0 = 2;
-constexpr int kEpilogueWarps = 16;
-constexpr int kThreads = 32 * (kEpilogueWarp0 + kEpilogueWarps);
 constexpr int kOperandBytes = kTileM * 128; // 16 KB of activations per stage: rows of 128 bytes of K
 constexpr int kMaxSlots = 4, kMaxStages = 6;
 constexpr int kBarrierBytes = 256;
@@ -67,10 +66,14 @@ constexpr int kBarrierBytes = 256;
 // dots each; a slot is handed over as a whole.
 template <bool F16, int TN> struct Form {
   static_assert(TN == 64 || TN == 96 || TN == 128, "tile widths with a tensor-memory plan");
+  static constexpr int kCtas = TN == 64 ? 2 : 1;                    // CTAs per SM
+  static constexpr int kEpilogueWarps = 16 / kCtas, kThreads = 32 * (kEpilogueWarp0 + kEpilogueWarps);
+  static constexpr int kTmemColumns = 512 / kCtas;
   static constexpr int kSlotBlocks = 2;
-  static constexpr int kSlots = 512 / (kSlotBlocks * TN);
-  static constexpr int kWarpColumns = TN / 4;                       // columns per epilogue warp: 16, 24 or 32
-  static constexpr int kStages = TN >= 128 ? 5 : 6;
+  static constexpr int kSlots = kTmemColumns / (kSlotBlocks * TN);
+  static constexpr int kWarpColumns = TN * 4 / kEpilogueWarps;      // columns per epilogue warp: 24 or 32
+  static constexpr int kStages = TN == 64 ? 4 : TN >= 128 ? 5 : 6;
+  static constexpr int kPiece = TN == 64 ? 16 : kWarpColumns;       // columns loaded from tensor memory at a time
   static constexpr int kStageBlocks = F16 ? 2 : 4;
   static constexpr int kStageK = kStageBlocks * 32;                 // elements of K per stage
   static constexpr int kOperandBytesB = TN * 128;
@@ -79,7 +82,7 @@ template <bool F16, int TN> struct Form {
   static constexpr int kCopied = kOperandBytes + kOperandBytesB + kScaleBytesA + kScaleBytesB;
   static constexpr int kStageBytes = (kCopied + 1023) / 1024 * 1024;
   static constexpr size_t kSmemBytes = 1024 + kStages * kStageBytes + kBarrierBytes;
-  static_assert(kSmemBytes <= 227 * 1024 && kSlots >= 2 && kSlots <= kMaxSlots, "plan of a CTA");
+  static_assert(kSmemBytes * kCtas <= 226 * 1024 && kSlots >= 2 && kSlots <= kMaxSlots, "plan of a CTA");
 };
 
 // kind::f16: f16 x f16 -> f32, both operands K-major, M = 128, N = TN, K = 16 per instruction.
@@ -154,13 +157,14 @@ static_assert(sizeof(Barriers) <= kBarrierBytes, "barriers");
 // fault (test hook): 1 = the loader announces the first stage's bytes but never issues its copies,
 // so the barrier of that stage cannot complete and every wait behind it has to run out.
 template <bool F16, bool DOTS, int TN>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(Form<F16, TN>::kThreads, Form<F16, TN>::kCtas)
 gemm_q8_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const __grid_constant__ CUtensorMap map_as, const __grid_constant__ CUtensorMap map_bs, int M, int K,
                     int N, int tiles, int m_tiles, void *__restrict__ y, int y_dtype, int activation,
                     int32_t *__restrict__ dots_out, int *__restrict__ error_out, uint32_t spin_limit, int fault) {
   using F = Form<F16, TN>;
   constexpr int kStageBlocks = F::kStageBlocks, kStages = F::kStages, kSlots = F::kSlots, kSlotBlocks = F::kSlotBlocks;
+  constexpr int kEpilogueWarps = F::kEpilogueWarps;
   constexpr int kColumns = F::kWarpColumns;
   extern __shared__ uint8_t raw_smem[];
   uint8_t *base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) & ~uintptr_t(1023));
@@ -186,7 +190,7 @@ gemm_q8_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_base)),
-                 "r"(512)
+                 "r"(F::kTmemColumns)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -309,33 +313,37 @@ gemm_q8_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
               break;
             tc_fence_after();
           }
-          uint32_t raw[kColumns];
-          tmem_load_columns<kColumns>(taddr0 + (slots.at * kSlotBlocks + j % kSlotBlocks) * TN, raw);
-          if (j % kSlotBlocks == kSlotBlocks - 1 || j == blocks - 1) {
-            // The slot is handed back before its last block is folded in.
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0)
-              mbar_arrive(&bars->tempty[slots.at]);
-            slots.next(kSlots);
-          }
           const float a_scale = scales[j * kTileM + row];
           const float4 *w_scale = reinterpret_cast<const float4 *>(scales + kStageBlocks * kTileM + j * TN + column0);
+          constexpr int kPiece = F::kPiece;
 #pragma unroll
-          for (int g = 0; g < kColumns / 4; ++g) {
-            const float4 w = w_scale[g];
-            float v[4];
+          for (int p = 0; p < kColumns; p += kPiece) {
+            uint32_t raw[kPiece];
+            tmem_load_columns<kPiece>(taddr0 + (slots.at * kSlotBlocks + j % kSlotBlocks) * TN + p, raw);
+            if (p + kPiece == kColumns && (j % kSlotBlocks == kSlotBlocks - 1 || j == blocks - 1)) {
+              // The slot is handed back before its last columns are folded in.
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0)
+                mbar_arrive(&bars->tempty[slots.at]);
+              slots.next(kSlots);
+            }
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-              v[u] = F16 ? __uint_as_float(raw[4 * g + u]) : __int2float_rn(static_cast<int>(raw[4 * g + u]));
-            fold2(acc[4 * g + 0], acc[4 * g + 1], v[0], v[1], a_scale, w.x, w.y);
-            fold2(acc[4 * g + 2], acc[4 * g + 3], v[2], v[3], a_scale, w.z, w.w);
-            if (DOTS && gm < M) {
+            for (int g = 0; g < kPiece / 4; ++g) {
+              const float4 w = w_scale[p / 4 + g];
+              float v[4];
 #pragma unroll
               for (int u = 0; u < 4; ++u)
-                if (gn0 + 4 * g + u < N)
-                  dots_out[(static_cast<size_t>(gm) * N + gn0 + 4 * g + u) * nb + it * kStageBlocks + j] =
-                      F16 ? __float2int_rn(v[u]) : static_cast<int>(raw[4 * g + u]);
+                v[u] = F16 ? __uint_as_float(raw[4 * g + u]) : __int2float_rn(static_cast<int>(raw[4 * g + u]));
+              fold2(acc[p + 4 * g + 0], acc[p + 4 * g + 1], v[0], v[1], a_scale, w.x, w.y);
+              fold2(acc[p + 4 * g + 2], acc[p + 4 * g + 3], v[2], v[3], a_scale, w.z, w.w);
+              if (DOTS && gm < M) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                  if (gn0 + p + 4 * g + u < N)
+                    dots_out[(static_cast<size_t>(gm) * N + gn0 + p + 4 * g + u) * nb + it * kStageBlocks + j] =
+                        F16 ? __float2int_rn(v[u]) : static_cast<int>(raw[4 * g + u]);
+              }
             }
           }
         }
@@ -379,7 +387,7 @@ gemm_q8_tma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(F::kTmemColumns) : "memory");
   }
   if (tid == 0 && bars->abort_flag && error_out)
     atomicExch(error_out, 1);
@@ -455,27 +463,22 @@ template <bool F16, int TN> cudaError_t launch_tile(const GemmCall &c) {
   const int64_t tiles = static_cast<int64_t>(m_tiles) * ((c.N + TN - 1) / TN);
   if (tiles >= (1 << 30))
     return cudaErrorInvalidValue;
-  launch_chained(kernel, dim3(static_cast<unsigned>(std::min<int64_t>(tiles, c.sm_count))), dim3(kThreads), F::kSmemBytes, c.stream,
+  launch_chained(kernel, dim3(static_cast<unsigned>(std::min<int64_t>(tiles, c.sm_count * F::kCtas))), dim3(F::kThreads), F::kSmemBytes, c.stream,
                  map_a, map_b, map_as, map_bs, c.M, c.K, c.N, static_cast<int>(tiles), m_tiles, c.y, c.y_dtype, c.activation,
                  c.dots_out, c.error_flag, c.spin_limit, c.fault);
   return cudaGetLastError();
 }
 
-// Tile width for an M x N output: a CTA works through ceil(tiles / SMs) tiles, each at a cost that grows with its
-// width and has a part that does not (the hand-off of a block, worth about 72 columns: 23.4, 27.8 and
-// 33.7 us for one tile of K = 2560).
+// Tile width for an M x N output: an SM works through ceil(tiles / SMs) tiles.  Measured per tile at K = 2560: 32.7 us
+// for 128 columns, 26.7 for 96; 64-column tiles run two to an SM, 34.5 us for both or 23.7 for one alone (1024 x 8192:
+// 119 us in 64 columns, 129 in 128; 1024 x 9216: 138 and 130; 517 x 8192: 88 in 64, 79 in 96).
 int choose_tile(int M, int N, int sm_count) {
   if (const int forced = gemm_forced_tile())
     return forced;
   const int64_t rows = (M + kTileM - 1) / kTileM;
-  int best = 128;
-  int64_t best_cost = INT64_MAX;
-  for (const int width : {128, 96, 64}) {
-    const int64_t tiles = rows * ((N + width - 1) / width), cost = (tiles + sm_count - 1) / sm_count * (width + 72);
-    if (cost < best_cost)
-      best = width, best_cost = cost;
-  }
-  return best;
+  auto per_sm = [&](int width) { return (rows * ((N + width - 1) / width) + sm_count - 1) / sm_count; };
+  const int64_t cost128 = per_sm(128) * 327, cost96 = per_sm(96) * 267, cost64 = per_sm(64) / 2 * 345 + per_sm(64) % 2 * 237;
+  return cost128 <= cost96 && cost128 <= cost64 ? 128 : cost96 <= cost64 ? 96 : 64;
 }
 
 template <bool F16> cudaError_t launch_form(const GemmCall &c) {
