@@ -155,6 +155,22 @@ def test_all_position_logits_match_oracle():
     engine.close()
 
 
+def test_all_position_logits_of_a_large_vocabulary():
+    """More logits than one staged copy holds (22 MB, a ragged last piece) reach the caller whole: each row against a
+    forward of its prefix, and a second call into the same engine; 44 rows also read their scales unrearranged."""
+    d = L.default_dims().copy(**dict(SMALL, vocab=131080))
+    engine = L.Engine(L.synthetic_container(d, 6), d, capacity=48)
+    prompt = np.random.default_rng(6).integers(0, d.vocab, size=44).tolist()
+    rows = engine.forward_all(prompt, 0)
+    assert rows.nbytes > 16 << 20 and rows.nbytes % (2 << 20) != 0
+    for s in (0, 1, 20, 42, 43):
+        engine.reset()
+        assert np.array_equal(rows[s].view(np.uint32), engine.forward(prompt[:s + 1], 0)[0].view(np.uint32)), s
+    engine.reset()
+    assert np.array_equal(engine.forward_all(prompt, 0).view(np.uint32), rows.view(np.uint32))
+    engine.close()
+
+
 def test_one_token_prompt_uses_decode_entry():
     d = L.default_dims().copy(**TINY)
     run_both(d, 3, [7], steps=3, capacity=8)  # AotRuntime.cpp:116: sequence == 1 -> decode entry
