@@ -519,12 +519,13 @@ int llmcp_op_linear_bf16(const uint16_t *x, int64_t M, int64_t K, const uint16_t
     Buf dx(static_cast<size_t>(M) * K * 2, x), dw(static_cast<size_t>(N) * K * 2, weight), dy(static_cast<size_t>(M) * N * elem(y_dtype)),
         dstatus(4);
     cuda_check(cudaMemset(dstatus.p, 0, 4), "memset");
-    if (M == 1)
-      cuda_check(launch_gemv_bf16(dx.as<uint16_t>(), static_cast<int>(K), dw.as<uint16_t>(), N, dy.p, y_dtype, activation, nullptr),
-                 "bf16 GEMV");
-    else
+    if (M == 1) {
+      const Bf16Job job = {dw.as<uint16_t>(), dy.p, N, y_dtype, activation};
+      cuda_check(launch_gemv_bf16(dx.as<uint16_t>(), static_cast<int>(K), &job, 1, nullptr), "bf16 GEMV");
+    } else {
       cuda_check(launch_gemm_bf16_tc(dx.as<uint16_t>(), static_cast<int>(M), static_cast<int>(K), dw.as<uint16_t>(),
                                      static_cast<int>(N), dy.p, y_dtype, activation, dstatus.as<int>(), nullptr), "bf16 GEMM");
+    }
     g_launches += 1;
     cuda_check(cudaDeviceSynchronize(), "bf16 linear");
     int status = 0;

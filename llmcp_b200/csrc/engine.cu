@@ -715,12 +715,20 @@ static void run_linears(const F16Planes &planes, const int8_t *aq, const float *
                         cudaStream_t stream, uint64_t *launches, int flags, int *gemm_error = nullptr,
                         const uint16_t *xb = nullptr, int *status = nullptr, const SideStreams *side = nullptr,
                         const PrefetchList *next = nullptr) {
-  if (jobs[0].w->bf) { // bf16 matrices: the input rows are bf16 (xb), one launch per matrix
+  if (jobs[0].w->bf) { // bf16 matrices: the input rows are bf16 (xb); one row: one launch for all, else one per matrix
+    if (S == 1) {
+      Bf16Job group[kMaxGemvJobs];
+      for (int i = 0; i < count; ++i)
+        group[i] = {jobs[i].w->bf, jobs[i].y, jobs[i].w->N, jobs[i].y_dtype, jobs[i].activation};
+      if (const cudaError_t e = launch_gemv_bf16(xb, jobs[0].w->K, group, count, stream); e != cudaSuccess)
+        throw std::runtime_error(std::string("bf16 linear: ") + cudaGetErrorString(e));
+      *launches += 1;
+      return;
+    }
     for (int i = 0; i < count; ++i) {
       const Q8Weight &w = *jobs[i].w;
-      const cudaError_t e = S == 1 ? launch_gemv_bf16(xb, w.K, w.bf, w.N, jobs[i].y, jobs[i].y_dtype, jobs[i].activation, stream)
-                                   : launch_gemm_bf16_tc(xb, static_cast<int>(S), w.K, w.bf, w.N, jobs[i].y, jobs[i].y_dtype,
-                                                         jobs[i].activation, status, stream);
+      const cudaError_t e = launch_gemm_bf16_tc(xb, static_cast<int>(S), w.K, w.bf, w.N, jobs[i].y, jobs[i].y_dtype, jobs[i].activation,
+                                                status, stream);
       if (e != cudaSuccess)
         throw std::runtime_error(std::string("bf16 linear: ") + cudaGetErrorString(e));
       *launches += 1;

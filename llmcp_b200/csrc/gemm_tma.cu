@@ -22,8 +22,8 @@
 // handing over every block by itself made it 1000.  Two blocks per hand-off, descriptors advanced by an add, one
 // elected lane per role (so that the compiler knows it is one) and a persistent grid (a tile's output is stored while
 // the next tile's blocks are already multiplied) bring it to 800: 1024 x 9216 x 2560 170 -> 130 us, 1024 x 2560 x 4096
-// 87 -> 84, 1024 x 32 x 2560 42 -> 22.  Fragment-shaped tensor-memory loads (16x256b: fewer scale registers) read
-// tensor memory at a quarter of the rate and measured 160 us.
+// 87 -> 84, 1024 x 32 x 2560 42 -> 22.  Tensor-memory loads in fragment shapes, which need a third of the scale
+// loads, measured 160 us (16x256b, a quarter of the read rate) and 150 us (16x128b, half).
 //
 // One CTA per SM (two of 320 threads for TN = 64, out of step with each other) takes 128 x TN output tiles in turn,
 // 576 threads:
@@ -34,12 +34,12 @@
 //               floats per block);
 //   warp  1     one lane issues the MMAs, two blocks into a tensor-memory slot (f16: two K = 16
 //               instructions per block, the first overwrites, the second accumulates), and commits the slot;
-//   warps 2-17  epilogue (2-9 for TN = 64): tcgen05.ld a block (thread = row, 24 or 32 columns), hand the slot back after its last
-//               block's load, then the arithmetic with the scales read from shared memory.
+//   warps 2-17  epilogue (2-9 for TN = 64): tcgen05.ld a block (thread = row, 24 or 32 columns), hand the slot back
+//               after its last block's load, then the arithmetic with the scales read from shared memory.
 // Hand-offs are mbarriers; every wait is bounded (spin_limit polls) and a timed-out wait raises an
 // abort flag that all roles observe, so a protocol error ends the kernel with an error code instead
 // of hanging it; the loader then waits (bounded) for the copies it has in flight.  Tensor memory
-// (512 columns) is allocated by warp 0 and always released.
+// (512 columns, half of it for TN = 64) is allocated by warp 0 and always released.
 
 #include <cuda.h>
 #include <cuda_fp16.h>

@@ -86,11 +86,11 @@ cudaError_t launch_gemm_q8_tc(const int8_t *aq, const float *as, int M, int K, c
 // row is written as zeros and the table is not read.
 // Tensor-core GEMM with TMA-fed operands (gemm_tma.cu).  Operand planes are [rows][K] and scale
 // planes block-major f32, [K/32][pitch] (pitch = gemm_tc16_scale_pitch(M) for activations, N for
-// weights); `form` says what the operand planes hold and how the epilogue multiplies:
+// weights); `form` says what the operand planes hold:
 //   kGemmI8  / kGemmI8Packed : int8 values, tcgen05 kind::i8, int32 dots converted in the epilogue;
 //   kGemmF16 / kGemmF16Packed: the same integers as f16 values, kind::f16, exact f32 dots;
-//   *Packed: two-lane f32x2 multiplies and fmas.
-// spin_limit 0 = default (about a second); fault: test hook, see the kernel.
+//   *Packed: the default of either kind; kGemmI8Packed also takes the narrow-tile kernel below.
+// spin_limit 0 = default (a few seconds); fault: test hook, see the kernel.
 enum GemmForm : int { kGemmI8 = 0, kGemmI8Packed = 1, kGemmF16 = 2, kGemmF16Packed = 3 };
 int64_t gemm_tc16_scale_pitch(int64_t M);
 void launch_act_to_f16(const int8_t *aq, const float *as, int64_t M, int K, void *ah, float *ast, cudaStream_t stream);
@@ -203,8 +203,14 @@ cudaError_t launch_attention_prepare(const uint16_t *qg, const uint16_t *k, cons
 // bf16 weights [N][K] of an unquantised arena (MatmulLoweringCommon.cpp:186-251): y = act(x w^T) with
 // f32 accumulation; one row through a streaming GEMV, more rows on the tensor cores (bf16 operands by
 // TMA; error_flag as for the Q8 GEMM).  GEMV: K % 16 == 0; GEMM: K % 8 == 0 and N % 8 == 0.
-cudaError_t launch_gemv_bf16(const uint16_t *x, int K, const uint16_t *w, int64_t N, void *y, int y_dtype, int activation,
-                             cudaStream_t stream);
+// Up to kMaxGemvJobs matrices that share the input row in one launch.
+struct Bf16Job {
+  const uint16_t *w; // [N][K]
+  void *y;
+  int64_t N;
+  int y_dtype, activation;
+};
+cudaError_t launch_gemv_bf16(const uint16_t *x, int K, const Bf16Job *jobs, int count, cudaStream_t stream);
 cudaError_t launch_gemm_bf16_tc(const uint16_t *x, int M, int K, const uint16_t *w, int N, void *y, int y_dtype, int activation,
                                 int *error_flag, cudaStream_t stream, uint32_t spin_limit = 0);
 cudaError_t launch_embedding_bf16(const int64_t *tokens, int64_t S, int H, int64_t vocab, const uint16_t *table, uint16_t *out,
