@@ -5,7 +5,6 @@
 #include <cstdlib>
 #include <cstring>
 #include <stdexcept>
-#include <system_error>
 #include <thread>
 
 #include "kernels.h"
@@ -1198,7 +1197,7 @@ void Engine::rows_to_host(float *host, const float *device, size_t bytes) {
     try {
       threads[w] = std::thread(work, w);
       started[w] = true;
-    } catch (const std::system_error &) { // no more threads: this one does that share below
+    } catch (...) { // no more threads: this one does that share below
     }
   }
   for (int w = 0; w < kWorkers; ++w)
