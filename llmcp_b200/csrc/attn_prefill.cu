@@ -392,7 +392,7 @@ cudaError_t launch_attention_prefill_tc(const uint16_t *qg, const uint16_t *k, c
   if (S <= 0 || !attention_prefill_tc_supported(nh, nkv, hd) || S > (1 << 24) || rot % 2 != 0 || rot > hd || max_position + S > cap)
     return cudaErrorInvalidValue;
   if (spin_limit == 0)
-    spin_limit = tc::kSpinLimit;
+    spin_limit = tc::kSpinLimit<true>;
   uint16_t *qn = static_cast<uint16_t *>(scratch);
   uint16_t *vt = reinterpret_cast<uint16_t *>(static_cast<unsigned char *>(scratch) + queries_bytes(S, nh));
   // q/k norms, rotary embedding and the cache rows of the new tokens: the exact path's kernel, tree sums

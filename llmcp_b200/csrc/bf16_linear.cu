@@ -223,7 +223,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       int issued = 0;
       for (int it = 0; it < slices; ++it) {
         const int s = it % kStages;
-        if (it >= kStages && !mbar_wait(&bars->empty[s], ((it / kStages) - 1) & 1, abort_flag, spin_limit))
+        if (it >= kStages && !mbar_wait<false>(&bars->empty[s], ((it / kStages) - 1) & 1, abort_flag, spin_limit))
           break;
         mbar_expect_tx(&bars->full[s], kStageBytes);
         issued = it + 1;
@@ -232,14 +232,14 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       }
       if (*abort_flag) // copies already requested still write into this CTA's shared memory
         for (int it = max(0, issued - kStages); it < issued; ++it)
-          mbar_wait_quiet(&bars->full[it % kStages], (it / kStages) & 1, spin_limit);
+          mbar_wait_quiet<false>(&bars->full[it % kStages], (it / kStages) & 1, spin_limit);
     }
   } else if (warp == 1) {
     if (lane == 0) {
       bool ok = true;
       for (int it = 0; it < slices && ok; ++it) {
         const int s = it % kStages;
-        ok = mbar_wait(&bars->full[s], (it / kStages) & 1, abort_flag, spin_limit);
+        ok = mbar_wait<false>(&bars->full[s], (it / kStages) & 1, abort_flag, spin_limit);
         if (!ok)
           break;
         tc_fence_after();
@@ -254,7 +254,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   } else {
     const int quarter = warp & 3; // tensor-memory lanes 32 * quarter .. + 31 (fixed by the warp number)
     const int gm = m0 + quarter * 32 + lane;
-    if (__all_sync(0xffffffffu, mbar_wait(&bars->done, 0, abort_flag, spin_limit))) {
+    if (__all_sync(0xffffffffu, mbar_wait<false>(&bars->done, 0, abort_flag, spin_limit))) {
       tc_fence_after();
 #pragma unroll 1
       for (int c = 0; c < kTile / 32; ++c) {
@@ -336,7 +336,7 @@ cudaError_t launch_gemm_bf16_tc(const uint16_t *x, int M, int K, const uint16_t 
   if (M <= 0 || N <= 0 || N % 8 != 0 || K <= 0 || K % 8 != 0)
     return cudaErrorInvalidValue;
   if (spin_limit == 0)
-    spin_limit = tc::kSpinLimit;
+    spin_limit = tc::kSpinLimit<false>;
   CUtensorMap map_x, map_w;
   if (!bf16_map(&map_x, x, M, K) || !bf16_map(&map_w, w, N, K))
     return cudaErrorNotSupported;

@@ -291,7 +291,7 @@ cudaError_t launch_gemm_q8_few(const int8_t *aq, const float *as, bool row_scale
   if (M <= 0 || N % 8 != 0 || K % kBlock != 0 || (row_scales && (dots_out || !gemm_few_takes_row_scales(M, K, as))))
     return cudaErrorInvalidValue;
   if (spin_limit == 0)
-    spin_limit = kSpinLimit;
+    spin_limit = kSpinLimit<true>;
   FewCall call = {aq, as, row_scales, M, K, wq, wst, N, y, y_dtype, activation, dots_out, error_flag, stream, spin_limit, fault, 148};
   int sms = 0;
   if (current_sm_count(&sms) == cudaSuccess && sms > 0)

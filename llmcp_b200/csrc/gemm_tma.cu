@@ -129,7 +129,7 @@ __device__ __forceinline__ void fold2(float &c0, float &c1, float v0, float v1, 
 
 // mbar_wait by a whole warp: all lanes get the same answer.
 __device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag, uint32_t limit) {
-  return __all_sync(0xffffffffu, mbar_poll(smem_u32(bar), parity)) ||
+  return __all_sync(0xffffffffu, mbar_poll<true>(smem_u32(bar), parity)) ||
          __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, limit));
 }
 
@@ -550,7 +550,7 @@ cudaError_t launch_gemm_q8_tma(int form, const void *a, const float *ast, int M,
   if (M <= 0 || N % 8 != 0 || K % kBlock != 0)
     return cudaErrorInvalidValue;
   if (spin_limit == 0)
-    spin_limit = tc::kSpinLimit;
+    spin_limit = tc::kSpinLimit<true>;
   GemmCall call = {a, ast, M, K, w, wst, N, y, y_dtype, activation, dots_out, error_flag, stream, spin_limit, fault, 148};
   int sms = 0;
   if (current_sm_count(&sms) == cudaSuccess && sms > 0)

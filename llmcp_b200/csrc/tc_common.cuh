@@ -33,28 +33,38 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
                : "memory");
 }
 
-// One bounded look at the phase with the given parity: the hardware may suspend the thread for up to kPollNs.  Without
-// the hint a poll returns after some 20 cycles, and the single lanes that wait most of the time (loader, MMA issue)
-// then took a third of an SM's issue slots and its instruction cache from the warps that compute.
+// One bounded look at the phase with the given parity.  SUSPEND: the hardware may put the thread to sleep for up to
+// kPollNs.  A poll without that returns after some 20 cycles, and the single lanes that wait most of the time (loader,
+// MMA issue) then take issue slots and instruction cache from the warps that compute; waking up costs a microsecond
+// over the serial stages of a kernel whose warps compute little (the bf16 GEMM: 28.9 us without, 29.9 with, per
+// projection of a short prompt).
 constexpr uint32_t kPollNs = 1000;
-constexpr uint32_t kSpinLimit = 1u << 21; // polls before a wait gives up, unless the caller says otherwise: seconds
-__device__ __forceinline__ bool mbar_poll(uint32_t addr, uint32_t parity) {
+// Polls before a wait gives up, unless the caller says otherwise: seconds in the first form, about one in the second.
+template <bool SUSPEND> constexpr uint32_t kSpinLimit = SUSPEND ? 1u << 21 : 1u << 26;
+template <bool SUSPEND> __device__ __forceinline__ bool mbar_poll(uint32_t addr, uint32_t parity) {
   uint32_t done;
-  asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }"
-               : "=r"(done)
-               : "r"(addr), "r"(parity), "r"(kPollNs)
-               : "memory");
+  if (SUSPEND)
+    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }"
+                 : "=r"(done)
+                 : "r"(addr), "r"(parity), "r"(kPollNs)
+                 : "memory");
+  else
+    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                 : "=r"(done)
+                 : "r"(addr), "r"(parity)
+                 : "memory");
   return done != 0;
 }
 
 // Waits for the phase with the given parity; gives up when `abort_flag` is raised or after `limit`
 // polls (and then raises it).  Returns false on failure.
+template <bool SUSPEND = true>
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag, uint32_t limit) {
   const uint32_t addr = smem_u32(bar);
   for (uint32_t spin = 0; spin < limit; ++spin) {
-    if (mbar_poll(addr, parity))
+    if (mbar_poll<SUSPEND>(addr, parity))
       return true;
-    if (*abort_flag)
+    if ((SUSPEND || (spin & 63) == 63) && *abort_flag)
       return false;
   }
   *abort_flag = 1;
@@ -62,10 +72,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
 }
 
 // The same wait without the abort protocol (used while leaving after an abort).
-__device__ __forceinline__ bool mbar_wait_quiet(uint64_t *bar, uint32_t parity, uint32_t limit) {
+template <bool SUSPEND = true> __device__ __forceinline__ bool mbar_wait_quiet(uint64_t *bar, uint32_t parity, uint32_t limit) {
   const uint32_t addr = smem_u32(bar);
   for (uint32_t spin = 0; spin < limit; ++spin)
-    if (mbar_poll(addr, parity))
+    if (mbar_poll<SUSPEND>(addr, parity))
       return true;
   return false;
 }
