@@ -21,8 +21,8 @@
 // conversion, scales and fmas alone take 430 cycles per 128 x 128 x 32 block on an SM (346 without the conversion);
 // handing over every block by itself made it 1000.  Two blocks per hand-off, descriptors advanced by an add, one
 // elected lane per role (so that the compiler knows it is one) and a persistent grid (a tile's output is stored while
-// the next tile's blocks are already multiplied) bring it to 800: 1024 x 9216 x 2560 170 -> 130 us, 1024 x 2560 x 4096
-// 87 -> 84, 1024 x 32 x 2560 42 -> 22.  Tensor-memory loads in fragment shapes, which need a third of the scale
+// the next tile's blocks are already multiplied) bring it to 800 (bf16 outputs): 1024 x 9216 x 2560 170 -> 130 us,
+// 1024 x 2560 x 4096 87 -> 84, 1024 x 32 x 2560 42 -> 22.  Tensor-memory loads in fragment shapes, which need a third of the scale
 // loads, measured 160 us (16x256b, a quarter of the read rate) and 150 us (16x128b, half).
 //
 // One CTA per SM (two of 320 threads for TN = 64, out of step with each other) takes 128 x TN output tiles in turn,
@@ -44,6 +44,8 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
+#include <cstdio>
+#include <cstdlib>
 #include <mutex>
 
 #include "kernels.h"
@@ -519,7 +521,14 @@ scales_block_major_kernel(const void *__restrict__ scales, int scales_are_f16, i
 int gemm_forced_tile() {
   const char *flag = std::getenv("LLMCP_B200_GEMM_TILE");
   const int forced = flag ? std::atoi(flag) : 0;
-  return forced == 64 || forced == 96 || forced == 128 ? forced : 0;
+  if (forced == 64 || forced == 96 || forced == 128)
+    return forced;
+  static std::once_flag told;
+  if (flag && *flag)
+    std::call_once(told, [flag] {
+      std::fprintf(stderr, "llmcp_b200: LLMCP_B200_GEMM_TILE=%s is not a tile width (64, 96 or 128): chosen per shape\n", flag);
+    });
+  return 0;
 }
 
 int64_t gemm_tc16_scale_pitch(int64_t M) { return (M + 3) / 4 * 4; }

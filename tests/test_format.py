@@ -2,7 +2,10 @@
 synthetic checkpoint, and the exported C ABI.  No GPU is needed."""
 import ctypes as C
 import json
+import os
 import re
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -16,6 +19,20 @@ TINY = dict(hidden=64, intermediate=96, vocab=256, layers=4, full_interval=4, he
 
 def tiny_dims(**changes):
     return L.default_dims().copy(**{**TINY, **changes})
+
+
+@pytest.mark.parametrize("value,width", [(None, 0), ("", 0), ("64", 64), ("96", 96), ("128", 128), ("160", 0), ("wide", 0)])
+def test_forced_gemm_tile_width(value, width):
+    """LLMCP_B200_GEMM_TILE: a width the GEMM does not have leaves the choice to the shape and says so, once."""
+    env = {k: v for k, v in os.environ.items() if k != "LLMCP_B200_GEMM_TILE"}
+    if value is not None:
+        env["LLMCP_B200_GEMM_TILE"] = value
+    code = ("import llmcp_b200 as L\nforced = L.lib()['_ZN10llmcp_b20016gemm_forced_tileEv']\n"
+            "assert forced() == forced() and not print(forced())")
+    run = subprocess.run([sys.executable, "-c", code], env=env, cwd=L._PACKAGE.parent, capture_output=True, text=True, timeout=120)
+    assert run.returncode == 0 and run.stdout.split() == [str(width)], run.stderr
+    told = [line for line in run.stderr.splitlines() if "LLMCP_B200_GEMM_TILE" in line]
+    assert len(told) == (1 if value and not width else 0), run.stderr
 
 
 def test_every_declared_symbol_is_exported():
