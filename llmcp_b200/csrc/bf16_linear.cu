@@ -24,7 +24,7 @@ namespace {
 using namespace tc;
 
 constexpr int kGemvRows = 2;
-constexpr int kGemvPieces = 4; // pieces of 16 weights per row and lane in flight
+constexpr int kGemvPieces = 5; // pieces of 16 weights per row and lane in flight
 constexpr int kGemvThreads = 128;
 
 struct Words8 {
@@ -53,10 +53,12 @@ __device__ __forceinline__ float dot16(const Words8 &w, const float *x) {
 // K % 16 == 0; pieces past the row's end count as zeros.  N need not be a multiple of kGemvRows.  A lane sums its pieces
 // of 16 in ascending order, each as a chain of fmas, then the lanes are added as a tree.
 //
-// Bound: HBM.  Every warp keeps kGemvRows x kGemvPieces loads of 32 bytes per lane in flight (8 KB), the first of them
+// Bound: HBM.  Every warp keeps kGemvRows x kGemvPieces loads of 32 bytes per lane in flight (10 KB), the first of them
 // requested before the kernel in front has finished (weights do not depend on it), and reads the input row from L1 as
-// it is, 32 bytes per lane.  With one piece per row in flight, a f32 copy of the row in shared memory and a barrier in
-// front of the first weight, a 200-token prompt and 32 steps took 137 ms; now 102 (model of 8.4 GB; same sums).
+// it is, 32 bytes per lane.  Two rows, so that 2560 rows fill the SMs; five pieces, so that a row of K = 2560 is one trip
+// (a second trip for its last piece alone: the vocabulary matrix 201 us, 179 so; 9216 x 2560 twice 18.4 and 17.3,
+// 2560 x 9216 12.7 and 11.8).  Four rows with one piece each in flight, a f32 copy of the input row in shared memory and
+// a barrier in front of the first weight: vocabulary matrix 184 us, 2560 x 9216 33 us.
 // The matrices of a launch share the input row; their row pairs are numbered one after the other (a matrix with an odd
 // row count ends in a pair of one).  A layer's four input projections are two of 32 rows beside two of thousands, and
 // each launch of a chain costs 2 us or more however small: one launch per group, 102 -> 92 ms for the 200-token

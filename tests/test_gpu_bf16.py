@@ -5,6 +5,8 @@ The reference lowers the bf16 sum differently per target (MatmulLoweringCommon.c
 253-330 BFDOT) and holds it to a tolerance in its own tests (tests/numeric/run_numeric.py:676-688:
 relative 2e-2, absolute 1e-2), so the bar here is a tolerance as well: against a plain f32 matrix
 product, and against the oracle's restatement of the portable lowering."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -42,9 +44,10 @@ def test_linear_bf16_against_f32_product(M, N, K):
         assert np.abs(got_b - act(want)).max() <= 2.0 ** -7 * max(1.0, np.abs(act(want)).max())  # one bf16 rounding
 
 
-@pytest.mark.parametrize("N,K", [(1, 16), (7, 48), (2, 512), (9, 528), (4737, 2064), (3, 12288)])
+@pytest.mark.parametrize("N,K", [(1, 16), (7, 48), (2, 512), (9, 528), (37, 2560), (38, 2576), (18947, 2576), (3, 12288)])
 def test_gemv_bf16_edges(N, K):
-    """One row: pieces past the row's end, odd row counts, more rows than warps in flight, the longest row."""
+    """One row: pieces past the row's end, rows of one trip and of one piece more, odd row counts, more pairs of rows than
+    the grid has warps (148 x 16 CTAs of four), the longest row."""
     torch = pytest.importorskip("torch")
     rng = np.random.default_rng(N + K)
     x, w = bf16(rng.standard_normal((1, K))), bf16(rng.standard_normal((N, K)) * 0.05)
@@ -52,6 +55,43 @@ def test_gemv_bf16_edges(N, K):
     magnitude = np.abs(f(x)).astype(np.float64) @ np.abs(f(w)).astype(np.float64).T
     # a lane adds K / 32 products and the lanes are added in five steps: |error| <= (K / 32 + 22) 2^-24 sum |x w|
     assert (np.abs(L.ops.linear_bf16(x, w, y_bf16=False) - want) <= (K / 32 + 22) * 2.0 ** -24 * magnitude).all()
+
+
+class Bf16Job(C.Structure):
+    _fields_ = [("w", C.c_void_p), ("y", C.c_void_p), ("N", C.c_int64), ("y_dtype", C.c_int), ("activation", C.c_int)]
+
+
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("K,rows", [(528, (33, 18931, 7, 1)), (2560, (1, 50)), (2576, (7, 33, 2, 5)), (64, (3,))])
+def test_gemv_bf16_matrices_in_one_launch(K, rows, offset):
+    """Matrices that share an input row, odd row counts in front of others, and the row at and off a 16-byte boundary: each
+    output has the bits of the matrix's own launch, and no other element is written."""
+    torch = pytest.importorskip("torch")
+    launch = getattr(L.lib(), "_ZN10llmcp_b20016launch_gemv_bf16EPKtiPKNS_7Bf16JobEiP11CUstream_st")
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    g = torch.Generator(device="cuda").manual_seed(K + len(rows))
+    x = torch.randn(K + 8, generator=g, device="cuda").to(torch.bfloat16)[offset:offset + K]
+    w = [torch.randn(n, K, generator=g, device="cuda").to(torch.bfloat16) for n in rows]
+    kinds = [(i % 2, i % 4) for i in range(len(rows))]  # output type, activation
+
+    def outputs():
+        return [torch.full((n + 1,), 7.0, dtype=torch.bfloat16 if b else torch.float32, device="cuda") for n, (b, _) in zip(rows, kinds)]
+
+    def run(ys, which):
+        jobs = (Bf16Job * len(which))(*[Bf16Job(w[i].data_ptr(), ys[i].data_ptr(), rows[i], *kinds[i]) for i in which])
+        assert launch(C.c_void_p(x.data_ptr()), K, jobs, len(which), stream) == 0
+
+    together, alone = outputs(), outputs()
+    run(together, range(len(rows)))
+    for i in range(len(rows)):
+        run(alone, [i])
+    torch.cuda.synchronize()
+    for i, n in enumerate(rows):
+        assert torch.equal(together[i], alone[i]), i
+        assert float(together[i][n]) == 7.0
+        if kinds[i] == (0, 0):
+            want, size = w[i].double() @ x.double(), w[i].double().abs() @ x.double().abs()
+            assert bool(((together[i][:n] - want).abs() <= (K / 32 + 22) * 2.0 ** -24 * size).all())
 
 
 def oracle_dims(d):
