@@ -49,6 +49,11 @@ int dtype_of(const TensorEntry &t) {
 
 std::atomic<int> g_default_mode{-1};
 
+// Rows of logits on their way to pageable host memory (rows_to_host): pinned slots, and from which size on they serve.
+constexpr size_t kStagePiece = 2u << 20;
+constexpr int kStageSlots = 8;
+bool stages(size_t bytes) { return bytes > (kStageSlots - 1) * kStagePiece; }
+
 } // namespace
 
 // Names of the prefill GEMM forms (LLMCP_B200_GEMM): the value is 0 for the CUDA-core kernel, 1 for
@@ -239,6 +244,8 @@ Engine::Engine(const uint8_t *base, uint64_t file_bytes, const ModelDims &dims, 
   generated_ = static_cast<int64_t *>(alloc(static_cast<size_t>(capacity_) * 8));
   check(cudaMallocHost(&logits_pinned_, static_cast<size_t>(c.vocab) * 4), "cudaMallocHost");
   check(cudaMallocHost(&token_pinned_, 16), "cudaMallocHost");
+  if (batch_ > 1 && stages(static_cast<size_t>(batch_) * dims_.vocab * 4)) // a step of decode_batch takes no pinned memory
+    take_stage();
   reset_state();
   ensure_workspace(1, capacity_ - 1);
   // One throw-away decode step loads every kernel and applies its launch attributes, so that
@@ -1150,40 +1157,50 @@ int64_t Engine::forward_host(const int64_t *tokens, int64_t S, int64_t position,
   return *token_pinned_;
 }
 
+void Engine::take_stage() noexcept {
+  if (stage_pinned_ || cudaMallocHost(&stage_pinned_, kStageSlots * kStagePiece) == cudaSuccess)
+    return;
+  stage_pinned_ = nullptr; // no pinned memory left: rows_to_host copies directly
+  cudaGetLastError();
+}
+
 // Many rows of logits into the caller's memory.  A copy to pageable memory goes through the driver's one staging thread,
-// which also takes the page faults of a fresh buffer: 160 rows (159 MB) took 35 ms.  Here several threads each move
-// pieces of 2 MB through a pinned slot of their own, so that the stream's copies run beside the stores and the faults:
-// about 5 ms.  Pinned destinations and small copies go directly.
+// which also takes the page faults of a fresh buffer.  Here several threads each move pieces of 2 MB through a pinned
+// slot of their own, so that the stream's copies run beside the stores and the faults.  forward_all of 160 rows (159 MB)
+// on a small model: 36 -> 9.5 ms into a fresh buffer, 10.9 -> 7.5 into a used one; a batch of 64: 4.3 -> 3.3.  No more
+// threads than the process may use cores, and they give way while their copy is under way (events that sleep: 17 ms).
+// The slots cost a first call 6 to 15 ms, beside the forward.  Pinned destinations and small copies go directly.
 void Engine::rows_to_host(float *host, const float *device, size_t bytes) {
-  constexpr size_t kPiece = 2u << 20;
-  constexpr int kWorkers = 8;
-  const size_t pieces = (bytes + kPiece - 1) / kPiece;
+  const int workers = static_cast<int>(std::min<unsigned>(kStageSlots, std::max(1u, std::thread::hardware_concurrency())));
+  const size_t pieces = (bytes + kStagePiece - 1) / kStagePiece;
   cudaPointerAttributes where{};
   const bool pinned = cudaPointerGetAttributes(&where, host) == cudaSuccess && where.type != cudaMemoryTypeUnregistered;
   cudaGetLastError(); // an unknown pointer is not an error here
-  if (!pinned && pieces >= kWorkers && !stage_pinned_ && cudaMallocHost(&stage_pinned_, kWorkers * kPiece) != cudaSuccess) {
-    stage_pinned_ = nullptr; // no pinned memory left: the direct copy below
-    cudaGetLastError();
-  }
-  if (pinned || pieces < kWorkers || !stage_pinned_) {
+  const bool staged = !pinned && workers > 1 && stages(bytes);
+  if (staged)
+    take_stage();
+  if (!staged || !stage_pinned_) {
     check(cudaMemcpyAsync(host, device, bytes, cudaMemcpyDeviceToHost, stream_), "logits to the host");
     return;
   }
   check(cudaStreamSynchronize(stream_), "logits"); // the workers wait for copies, not for the forward
-  cudaError_t errors[kWorkers] = {};
+  cudaError_t errors[kStageSlots] = {};
   auto work = [&](int w) {
     cudaEvent_t arrived = nullptr;
     cudaError_t e = cudaSetDevice(device_);
     if (e == cudaSuccess)
       e = cudaEventCreateWithFlags(&arrived, cudaEventDisableTiming);
-    unsigned char *slot = stage_pinned_ + static_cast<size_t>(w) * kPiece;
-    for (size_t i = static_cast<size_t>(w); i < pieces && e == cudaSuccess; i += kWorkers) {
-      const size_t at = i * kPiece, n = std::min(kPiece, bytes - at);
+    unsigned char *slot = stage_pinned_ + static_cast<size_t>(w) * kStagePiece;
+    for (size_t i = static_cast<size_t>(w); i < pieces && e == cudaSuccess; i += static_cast<size_t>(workers)) {
+      const size_t at = i * kStagePiece, n = std::min(kStagePiece, bytes - at);
       e = cudaMemcpyAsync(slot, reinterpret_cast<const unsigned char *>(device) + at, n, cudaMemcpyDeviceToHost, stream_);
       if (e == cudaSuccess)
         e = cudaEventRecord(arrived, stream_);
-      if (e == cudaSuccess)
-        e = cudaEventSynchronize(arrived);
+      while (e == cudaSuccess && (e = cudaEventQuery(arrived)) == cudaErrorNotReady) {
+        cudaGetLastError(); // "not ready" is no error
+        std::this_thread::yield();
+        e = cudaSuccess;
+      }
       if (e == cudaSuccess)
         std::memcpy(reinterpret_cast<unsigned char *>(host) + at, slot, n);
     }
@@ -1191,19 +1208,19 @@ void Engine::rows_to_host(float *host, const float *device, size_t bytes) {
       cudaEventDestroy(arrived);
     errors[w] = e;
   };
-  std::thread threads[kWorkers];
-  bool started[kWorkers] = {};
-  for (int w = 1; w < kWorkers; ++w) {
+  std::thread threads[kStageSlots];
+  bool started[kStageSlots] = {};
+  for (int w = 1; w < workers; ++w) {
     try {
       threads[w] = std::thread(work, w);
       started[w] = true;
     } catch (...) { // no more threads: this one does that share below
     }
   }
-  for (int w = 0; w < kWorkers; ++w)
+  for (int w = 0; w < workers; ++w)
     if (!started[w])
       work(w);
-  for (int w = 1; w < kWorkers; ++w)
+  for (int w = 1; w < workers; ++w)
     if (started[w])
       threads[w].join();
   for (const cudaError_t e : errors)

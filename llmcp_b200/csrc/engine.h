@@ -231,7 +231,8 @@ private:
   float *logits_pinned_ = nullptr;
   int64_t *token_pinned_ = nullptr;
   void rows_to_host(float *host, const float *device, size_t bytes); // complete once the stream is synchronised
-  unsigned char *stage_pinned_ = nullptr;                            // rows_to_host, made by the first call that needs it
+  void take_stage() noexcept;
+  unsigned char *stage_pinned_ = nullptr; // rows_to_host: made with a batch engine whose steps need it, else by the first such call
   int64_t *position_dev_ = nullptr; // device scalar: start position of the running call
   // Inputs of the one-token step behind position_dev_ in one device block: token, cos row, sin row.
   int64_t *dec_tokens_ = nullptr;

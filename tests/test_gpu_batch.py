@@ -100,6 +100,32 @@ def test_batch_fast_mode_stays_close():
     assert r["worst"] <= 0.2, r["worst"]  # rounding-order differences only
 
 
+def test_batch_step_with_logits_takes_no_pinned_memory():
+    """33 sequences with 17 MB of logits per step: the slots that the logits pass through are taken with the engine, so the
+    first step that asks for logits leaves the process's shared resident memory (where pinned pages count) as it was; its
+    logits are those of a second step from the same state, whatever buffer they go to."""
+    d = L.default_dims().copy(**dict(SMALL, vocab=131080))
+    data = L.synthetic_container(d, 9)
+    engine = L.Engine(data, d, capacity=8, batch=33)
+    tokens = np.random.default_rng(9).integers(0, d.vocab, 33)
+
+    def shared_kb():
+        with open("/proc/self/status") as status:
+            return next(int(line.split()[1]) for line in status if line.startswith("RssShmem"))
+
+    engine.decode_batch(tokens, 0, want_logits=False)  # workspaces, kernels
+    engine.reset()
+    before = shared_kb()
+    logits, argmax = engine.decode_batch(tokens, 0)
+    grown = shared_kb() - before
+    assert grown < 1024, f"{grown} KB"
+    engine.reset()
+    again, _ = engine.decode_batch(tokens, 0)
+    assert np.array_equal(logits.view(np.uint32), again.view(np.uint32))
+    assert np.array_equal(logits.argmax(axis=1), argmax)
+    engine.close()
+
+
 def test_batch_engine_rejects_misuse():
     d = L.default_dims().copy(**TINY)
     data = L.synthetic_container(d, 1)
