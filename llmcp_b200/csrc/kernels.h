@@ -151,7 +151,10 @@ cudaError_t launch_gated_delta_net(const uint16_t *conv, const uint16_t *a, cons
                                    int a_log_dtype, const void *dt_bias, int dt_dtype, float *state, int64_t S,
                                    int nk, int nv, int dk, int dv, int b_activated, float *scratch,
                                    uint16_t *out, cudaStream_t stream, int ab_stride = 0 /* row pitch of a and b; 0 = nv */,
-                                   int fast = 0 /* S > 1, dk = 128: row quarters per lane, fused multiply-adds */);
+                                   int fast = 0 /* S > 1, dk = 128: sixteen rows of two columns per lane, fused multiply-adds */);
+// Loads the code of every kernel that launch_gated_delta_net chooses among in exact mode (by token count, sizes and the
+// inputs' alignment), for callers that must not meet a kernel's first launch later.
+cudaError_t load_gated_delta_net_kernels();
 // A batch of independent sequences, one token each, through the one-token kernels: element strides
 // between consecutive sequences' buffers (inputs and outputs are rows of a [sequences, width] matrix).
 struct GdnBatch {

@@ -734,6 +734,19 @@ size_t gdn_scratch_floats(int64_t S, int nk, int nv, int dk) {
   return static_cast<size_t>(S) * (2 * static_cast<size_t>(nk) * dk + 2 * static_cast<size_t>(nv));
 }
 
+cudaError_t load_gated_delta_net_kernels() {
+  const void *kernels[] = {reinterpret_cast<const void *>(gdn_prepare_kernel),
+                           reinterpret_cast<const void *>(gdn_recurrence_split_kernel<128, true>),
+                           reinterpret_cast<const void *>(gdn_recurrence_pipelined_kernel<128>),
+                           reinterpret_cast<const void *>(gdn_recurrence_kernel<128>),
+                           reinterpret_cast<const void *>(gdn_recurrence_kernel<0>)};
+  cudaFuncAttributes attributes;
+  for (const void *kernel : kernels)
+    if (const cudaError_t e = cudaFuncGetAttributes(&attributes, kernel); e != cudaSuccess)
+      return e;
+  return cudaSuccess;
+}
+
 cudaError_t launch_gated_delta_net(const uint16_t *conv, const uint16_t *a, const uint16_t *b,
                                    const void *a_log, int a_log_dtype, const void *dt_bias, int dt_dtype,
                                    float *state, int64_t S, int nk, int nv, int dk, int dv,

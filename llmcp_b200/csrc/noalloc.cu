@@ -16,8 +16,9 @@
 //     left there; the kernels write every element they later read, so nothing has to be
 //     cleared first.  Two calls that are in flight on the same GPU at the same time (two
 //     streams, two threads) would overwrite each other's vectors: keep them ordered;
-//   * the first call on each device looks up the array's device address.  Make that first
-//     call during start-up, before any stream capture is begun.
+//   * the first call on each device looks up the array's device address and loads the code of
+//     every kernel that a later call may choose (by token count, sizes and alignment).  Make
+//     that first call during start-up, before any stream capture is begun.
 
 #include <mutex>
 #include <string>
@@ -54,6 +55,11 @@ float *scratch_for_current_device(std::string *error) {
     e = cudaGetSymbolAddress(&address, g_gdn_scratch);
     if (e != cudaSuccess || !address) {
       *error = std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e);
+      return nullptr;
+    }
+    e = llmcp_b200::load_gated_delta_net_kernels();
+    if (e != cudaSuccess) {
+      *error = std::string("loading the gated_delta_net kernels: ") + cudaGetErrorString(e);
       return nullptr;
     }
     g_scratch_address[device] = static_cast<float *>(address);

@@ -9,6 +9,8 @@ be bit-identical to the allocating entry point's and to the CPU oracle's.  This 
 last on purpose.
 """
 import ctypes as C
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -104,6 +106,42 @@ def test_noalloc_leaves_free_device_memory_unchanged():
         for (S, nk, nv, dk, dv), (dev, out) in zip(shapes, held):
             assert _call(torch, dev, out, S, nk, nv, dk, dv) == 0
     assert torch.cuda.mem_get_info()[0] == free_before
+
+
+def test_noalloc_start_up_call_loads_what_a_capture_needs():
+    """In a fresh process one call of one token is the whole start-up: calls of several tokens, at and off a 16-byte
+    boundary (two kernels), are then made for the first time inside a stream capture, and the graph gives their results."""
+    code = """
+import sys; sys.path.insert(0, "tests")
+import numpy as np, torch, ctypes as C
+import llmcp_b200 as L, test_zz_no_alloc as T
+shape = (5, 2, 4, 128, 128)
+S, nk, nv, dk, dv = shape
+x = T._inputs(np.random.default_rng(8), *shape)
+dev, out = T._upload(torch, x, S, nv, dv)
+one, one_out = T._upload(torch, T._inputs(np.random.default_rng(9), 1, *shape[1:]), 1, nv, dv)
+assert T._call(torch, one, one_out, 1, *shape[1:]) == 0
+shifted = torch.empty(dev["conv"].numel() + 1, dtype=torch.int16, device="cuda")
+shifted[1:] = dev["conv"].reshape(-1)
+state, outs = dev["state"].clone(), [torch.zeros_like(out), torch.zeros_like(out)]
+states = [state.clone(), state.clone()]
+torch.cuda.synchronize()
+graph, p = torch.cuda.CUDAGraph(), lambda t: C.c_void_p(t.data_ptr())
+with torch.cuda.graph(graph):
+    for conv, o, s in ((dev["conv"], outs[0], states[0]), (shifted[1:], outs[1], states[1])):
+        assert L.lib().llmcp_dev_gated_delta_net_noalloc(
+            p(conv), p(dev["a"]), p(dev["b"]), p(dev["a_log"]), p(dev["dt_bias"]), p(s), *(C.c_int64(v) for v in shape), 0, p(o),
+            C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0, L.last_error()
+graph.replay()
+torch.cuda.synchronize()
+import oracle
+want, want_state = oracle.gated_delta_net(x["conv"], x["a"], x["b"], x["a_log"], x["dt_bias"], x["state"], nk, nv, dk, dv)
+for o, s in zip(outs, states):
+    assert np.array_equal(o.cpu().numpy().view(np.uint16), want)
+    assert np.array_equal(s.cpu().numpy().view(np.uint32), want_state.view(np.uint32))
+"""
+    run = subprocess.run([sys.executable, "-c", code], cwd=L._PACKAGE.parent, capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stderr
 
 
 def test_noalloc_rejects_oversized_calls():
