@@ -159,17 +159,18 @@ int llmcp_op_attention(const uint16_t *qg, const uint16_t *k, const uint16_t *v,
  *                         caller reads it after synchronising.
  *   llmcp_dev_gemm_q8_tma: the M > 1 linear on the tensor cores with operands fetched by TMA
  *                         (cp.async.bulk.tensor, no multicast).  form: 0 int8 operand planes,
- *                         tcgen05 kind::i8, int32 dots converted in the epilogue; 2 the same integers
- *                         held as f16 values, kind::f16 (an f16 x f16 block dot of int8-valued operands
- *                         is an exact integer in f32, so the result is the same bit for bit and the
- *                         conversion disappears); 1 and 3: the same with two-lane f32x2 multiplies and
- *                         fmas.  a / w: [rows][K] int8 (forms 0, 1) or f16 (2, 3); a_scales / w_scales:
+ *                         tcgen05 kind::i8, int32 dots converted in the epilogue; 1 the same, but few
+ *                         rows or few weight rows go to a kernel of narrow tiles (mma.sync, no tensor
+ *                         memory); 2 and 3, one kernel: the same integers held as f16 values, kind::f16
+ *                         (an f16 x f16 block dot of int8-valued operands is an exact integer in f32, so
+ *                         the conversion disappears).  Every form gives the same bits.
+ *                         a / w: [rows][K] int8 (forms 0, 1) or f16 (2, 3); a_scales / w_scales:
  *                         block-major f32 [K/32][pitch], pitch = llmcp_dev_gemm_q8_tma_scale_pitch(M)
  *                         (M rounded up to 4) for activations and N for weights.  status as above.
- *                         spin_limit: polls before a wait inside the kernel gives up (0 = default,
- *                         about a second).  fault: 0; 1 is a test hook that withholds the first
- *                         stage's copies so that the bounded waits run out (status becomes 1, y is
- *                         left unwritten, tensor memory is released).
+ *                         spin_limit: polls before a wait inside the kernel gives up, each up to a
+ *                         microsecond long (0 = default, a few seconds).  fault: 0; 1 is a test hook that
+ *                         withholds the first stage's copies so that the bounded waits run out (status
+ *                         becomes 1, y is left unwritten, tensor memory is released).
  *   llmcp_dev_q8_gemm_planes: those planes from int8 values [rows][K] and their scales
  *                         [rows][K/32] (f32 for activations, f16 bits for weights when
  *                         scales_are_f16): scales_block_major always, values_f16 if not null.
@@ -208,7 +209,7 @@ int llmcp_dev_argmax(const float *x, int64_t n, float *scratch_values, int64_t *
  * loads it): calls with S * (2*nk*dk + 2*nv) > 65536 are refused with code 2 and a message.
  * All calls on a GPU share that array, so calls that overlap in time on one GPU race; its
  * old contents need no clearing.  The first call on each device resolves the array's device
- * address; make it before starting any stream capture.  Calls no cudaMalloc / cudaFree. */
+ * address and loads the kernels; make it before starting any stream capture.  Calls no cudaMalloc / cudaFree. */
 int llmcp_dev_gated_delta_net_noalloc(const uint16_t *conv, const uint16_t *a, const uint16_t *b,
                                       const float *a_log, const uint16_t *dt_bias, float *state, int64_t S,
                                       int64_t nk, int64_t nv, int64_t dk, int64_t dv, int b_activated,

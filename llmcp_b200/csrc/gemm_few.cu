@@ -69,10 +69,10 @@ __device__ __forceinline__ void fold2(float &c0, float &c1, int d0, int d1, floa
       : "f"(s.x), "f"(s.y), "f"(w), "f"(__int2float_rn(d0)), "f"(__int2float_rn(d1)));
 }
 
-// fault (test hook): 1 = the producer announces the first stage's bytes but never issues its copies.
 __device__ __forceinline__ float component(float4 v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
 
 // ROWS: the activations' scales come as they are quantised, [M][K/32]; otherwise block-major.
+// fault (test hook): 1 = the producer announces the first stage's bytes but never issues its copies.
 template <int WN, int WM, int NT, int KS, int STAGES, bool DOTS, bool ROWS>
 __global__ void __launch_bounds__(Few<WN, WM, NT, KS, STAGES>::kThreads, 2)
 gemm_q8_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,

@@ -424,7 +424,7 @@ def _tma_gemm_setup(torch, M, N, K, seed):
     assert lib.llmcp_dev_q8_gemm_planes(None, ptr(wd), 1, C.c_int64(N), C.c_int64(K), None, ptr(wst2), stream) == 0
     torch.cuda.synchronize()
     assert torch.equal(ast2, ast) and torch.equal(wst2, wst)
-    return lib, stream, ptr, {"aq": aq, "wq": wq, "ah": ah, "wh": wh, "ast": ast, "wst": wst}, want
+    return lib, stream, ptr, {"aq": aq, "as": scales, "wq": wq, "ah": ah, "wh": wh, "ast": ast, "wst": wst}, want
 
 
 def _tma_gemm(lib, stream, ptr, planes, form, M, N, K, y, status, spin_limit=0, fault=0):
@@ -449,13 +449,17 @@ def test_gemm_tma_device_entry(M, N, K):
         assert np.array_equal(y.cpu().numpy().view(np.uint32), want.view(np.uint32)), form
 
 
+@pytest.mark.parametrize("tile", ["64", "96", "128"])
 @pytest.mark.parametrize("form", [1, 3])
-def test_gemm_tma_bounded_wait_runs_out_and_recovers(form):
+def test_gemm_tma_bounded_wait_runs_out_and_recovers(monkeypatch, form, tile):
     """The test hook withholds the first stage's copies: every wait behind it must give up after its
     bounded number of polls, the kernel must report through the status word, write nothing, free
-    its tensor memory and leave the context usable: the next launch is correct."""
+    its tensor memory and leave the context usable: the next launch is correct.  Every tile width
+    (a forced width is the tcgen05 kernel), with more tiles than CTAs."""
     torch = pytest.importorskip("torch")
-    M, N, K = 256, 384, 2560
+    M, N, K = 300, 8200, 608
+    assert 3 * ((N + int(tile) - 1) // int(tile)) > (2 if tile == "64" else 1) * torch.cuda.get_device_properties(0).multi_processor_count
+    monkeypatch.setenv("LLMCP_B200_GEMM_TILE", tile)
     lib, stream, ptr, planes, want = _tma_gemm_setup(torch, M, N, K, 99)
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
     y = torch.full((M, N), 7.0, dtype=torch.float32, device="cuda")
@@ -487,11 +491,10 @@ def test_linear_q8_every_gemm_form(monkeypatch):
         assert np.array_equal(dots, want_dots), form
 
 
-def test_linear_q8_both_tile_widths(monkeypatch):
-    """The TMA-fed GEMM with 128- and with 160-column tiles (the second exists for matrices whose
-    128-wide tiles would leave a nearly empty last wave): every form exact, block dots included, a
+def test_linear_q8_tile_widths(monkeypatch):
+    """The TMA-fed GEMM with 64-, 96- and 128-column tiles: every form exact, block dots included, a
     partial last tile in both directions, bf16 output with an activation; and the automatic choice on
-    a 1024 x 2560 output (160 tiles of 128 columns against 128 tiles of 160 in one wave)."""
+    a 1024 x 2560 output (160 tiles of 128 columns, 216 of 96)."""
     rng = np.random.default_rng(33)
     M, N, K = 130, 264, 2560
     packed = oracle.pack_q8_0_p4((rng.standard_normal((N, K)) * 0.02).astype(np.float32))
@@ -500,7 +503,7 @@ def test_linear_q8_both_tile_widths(monkeypatch):
     want_silu = oracle.linear_q8(x, packed, N, activation="silu")
     q, _ = oracle.act_quant(x)
     want_dots = oracle.block_dots(q, packed, N)
-    for tile in ("128", "160"):
+    for tile in ("64", "96", "128"):
         monkeypatch.setenv("LLMCP_B200_GEMM_TILE", tile)
         for form in ("i8", "i8x2", "f16", "f16x2"):
             monkeypatch.setenv("LLMCP_B200_GEMM", form)
@@ -519,20 +522,59 @@ def test_linear_q8_both_tile_widths(monkeypatch):
 
 
 
+def _few_preferred(lib, M, N):
+    """Whether the default form sends this shape to the narrow-tile kernel (gemm_few_preferred)."""
+    import ctypes as C
+    rule = lib["_ZN10llmcp_b20018gemm_few_preferredEii"]
+    rule.restype = C.c_bool
+    return rule(M, N)
+
+
+# The widths are 16, 32 or 64 weight rows by 32 (up to 32 rows) or 64; the last three of a list have more tiles than a
+# grid of two CTAs per SM (148), so that a CTA's ring of stages runs on into a second tile.
 @pytest.mark.parametrize("M,N,K", [(2, 8, 32), (32, 16, 2560), (33, 72, 96), (64, 2568, 288), (65, 136, 160), (7, 9216, 128),
-                                   (128, 2560, 4096), (300, 32, 2560), (1024, 40, 608), (64, 38016, 64), (40, 4104, 544)])
+                                   (128, 2560, 4096), (300, 32, 2560), (1024, 40, 608), (40, 4104, 544), (20, 4096, 2560),
+                                   (32, 9216, 2560), (17, 19016, 1184), (32, 19016, 64), (64, 19016, 832)])
 def test_gemm_few_rows(M, N, K):
     """The narrow-tile form of the default GEMM: bit-identical to the oracle at the edges of its tiles (16, 32 and 64
     weight rows, 32 and 64 rows), with a last stage that is not full, over several tiles per CTA, f32 and bf16 out."""
     import ctypes as C
     torch = pytest.importorskip("torch")
     lib, stream, ptr, planes, want = _tma_gemm_setup(torch, M, N, K, M + N + K)
+    assert _few_preferred(lib, M, N), "the rule sends this shape to another kernel: the case tests nothing here"
+    assert N < 19000 or (N + 63) // 64 > 2 * torch.cuda.get_device_properties(0).multi_processor_count
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
     y = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
     _tma_gemm(lib, stream, ptr, planes, 1, M, N, K, y, status)
     yb = torch.zeros((M, N), dtype=torch.bfloat16, device="cuda")
     assert lib.llmcp_dev_gemm_q8_tma(1, ptr(planes["aq"]), ptr(planes["ast"]), C.c_int64(M), C.c_int64(K), ptr(planes["wq"]),
                                      ptr(planes["wst"]), C.c_int64(N), ptr(yb), 1, 0, ptr(status), C.c_uint32(0), 0, stream) == 0
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    assert np.array_equal(y.cpu().numpy().view(np.uint32), want.view(np.uint32))
+    assert torch.equal(yb, torch.from_numpy(want).to(torch.bfloat16).cuda())
+
+
+@pytest.mark.parametrize("M,N,K", [(33, 72, 384), (63, 136, 1408), (130, 40, 640), (40, 4104, 128), (40, 4104, 1408), (63, 4096, 384),
+                                   (200, 2568, 128), (64, 9216, 896), (33, 19016, 896), (64, 19016, 128)])
+def test_gemm_few_rows_with_scales_as_quantised(M, N, K):
+    """The narrow-tile form on the activations' scales as the quantising kernels write them, [M][K/32]: the bits of the
+    oracle, with the last stage of 256 bytes of K half full (K = 384, 640, 1408), rings that wrap and, for the widest
+    matrices, more tiles than CTAs; what it cannot read is refused."""
+    import ctypes as C
+    torch = pytest.importorskip("torch")
+    lib, stream, ptr, planes, want = _tma_gemm_setup(torch, M, N, K, M + N + K)
+    launch = lib["_ZN10llmcp_b20018launch_gemm_q8_fewEPKaPKfbiiS1_S3_iPviiPiS5_P11CUstream_stji"]
+
+    def call(y, y_bf16, rows=M):
+        return launch(ptr(planes["aq"]), ptr(planes["as"]), C.c_bool(True), rows, K, ptr(planes["wq"]), ptr(planes["wst"]), N,
+                      ptr(y), y_bf16, 0, None, ptr(status), stream, C.c_uint32(0), 0)
+
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    y = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
+    yb = torch.zeros((M, N), dtype=torch.bfloat16, device="cuda")
+    assert call(y, 0) == 0 and call(yb, 1) == 0
+    assert call(y, 0, rows=32) != 0  # up to 32 rows read them block-major
     torch.cuda.synchronize()
     assert int(status.item()) == 0
     assert np.array_equal(y.cpu().numpy().view(np.uint32), want.view(np.uint32))
