@@ -1100,12 +1100,18 @@ uint64_t llmcp_b200_manifest(const uint8_t *file, uint64_t file_bytes, char *buf
   return bytes;
 }
 
+// Engines of this interface can be asked for the logits of many rows; an AOT session is not.
+static void *with_stage(Engine *engine) {
+  engine->prepare_rows_to_host();
+  return engine;
+}
+
 void *llmcp_b200_engine_create(const uint8_t *file, uint64_t file_bytes, const llmcp_b200_dims *dims, int64_t capacity,
                                int device) {
   try {
     const ModelDims d = to_dims(dims);
     check_dims(d);
-    return new Engine(file, file_bytes, d, capacity, device);
+    return with_stage(new Engine(file, file_bytes, d, capacity, device));
   } catch (const std::exception &e) {
     set_error(e.what());
     return nullptr;
@@ -1119,7 +1125,7 @@ void *llmcp_b200_engine_create_mode(const uint8_t *file, uint64_t file_bytes, co
     check_dims(d);
     if (mode != kModeExact && mode != kModeFast)
       throw std::runtime_error("mode must be 0 (exact) or 1 (fast)");
-    return new Engine(file, file_bytes, d, capacity, device, mode);
+    return with_stage(new Engine(file, file_bytes, d, capacity, device, mode));
   } catch (const std::exception &e) {
     set_error(e.what());
     return nullptr;
@@ -1166,7 +1172,7 @@ void *llmcp_b200_engine_create_tp(const uint8_t *file, uint64_t file_bytes, cons
     check_dims(d);
     if (mode != kModeExact && mode != kModeFast)
       throw std::runtime_error("mode must be 0 (exact) or 1 (fast)");
-    return new Engine(file, file_bytes, d, capacity, device, mode, static_cast<TpComm *>(tp), max_tokens);
+    return with_stage(new Engine(file, file_bytes, d, capacity, device, mode, static_cast<TpComm *>(tp), max_tokens));
   } catch (const std::exception &e) {
     set_error(e.what());
     return nullptr;
@@ -1180,7 +1186,7 @@ void *llmcp_b200_engine_create_batch(const uint8_t *file, uint64_t file_bytes, c
     check_dims(d);
     if (mode != kModeExact && mode != kModeFast)
       throw std::runtime_error("mode must be 0 (exact) or 1 (fast)");
-    return new Engine(file, file_bytes, d, capacity, device, mode, nullptr, 1024, batch);
+    return with_stage(new Engine(file, file_bytes, d, capacity, device, mode, nullptr, 1024, batch));
   } catch (const std::exception &e) {
     set_error(e.what());
     return nullptr;

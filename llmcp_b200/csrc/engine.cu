@@ -244,8 +244,6 @@ Engine::Engine(const uint8_t *base, uint64_t file_bytes, const ModelDims &dims, 
   generated_ = static_cast<int64_t *>(alloc(static_cast<size_t>(capacity_) * 8));
   check(cudaMallocHost(&logits_pinned_, static_cast<size_t>(c.vocab) * 4), "cudaMallocHost");
   check(cudaMallocHost(&token_pinned_, 16), "cudaMallocHost");
-  if (batch_ > 1 && stages(static_cast<size_t>(batch_) * dims_.vocab * 4)) // a step of decode_batch takes no pinned memory
-    take_stage();
   reset_state();
   ensure_workspace(1, capacity_ - 1);
   // One throw-away decode step loads every kernel and applies its launch attributes, so that
@@ -1164,12 +1162,17 @@ void Engine::take_stage() noexcept {
   cudaGetLastError();
 }
 
+void Engine::prepare_rows_to_host() noexcept {
+  if (stages(static_cast<size_t>(std::max<int64_t>(batch_, capacity_)) * dims_.vocab * sizeof(float)))
+    take_stage();
+}
+
 // Many rows of logits into the caller's memory.  A copy to pageable memory goes through the driver's one staging thread,
 // which also takes the page faults of a fresh buffer.  Here several threads each move pieces of 2 MB through a pinned
 // slot of their own, so that the stream's copies run beside the stores and the faults.  forward_all of 160 rows (159 MB)
 // on a small model: 36 -> 9.5 ms into a fresh buffer, 10.9 -> 7.5 into a used one; a batch of 64: 4.3 -> 3.3.  No more
-// threads than the process may use cores, and they give way while their copy is under way (events that sleep: 17 ms).
-// The slots cost a first call 6 to 15 ms, beside the forward.  Pinned destinations and small copies go directly.
+// threads than the process may use cores; they wait for their copies as the driver sees fit (it spins while there are
+// cores to spare; events that sleep made the 9.5 ms 17).  Pinned destinations and small copies go directly.
 void Engine::rows_to_host(float *host, const float *device, size_t bytes) {
   const int workers = static_cast<int>(std::min<unsigned>(kStageSlots, std::max(1u, std::thread::hardware_concurrency())));
   const size_t pieces = (bytes + kStagePiece - 1) / kStagePiece;
@@ -1196,11 +1199,8 @@ void Engine::rows_to_host(float *host, const float *device, size_t bytes) {
       e = cudaMemcpyAsync(slot, reinterpret_cast<const unsigned char *>(device) + at, n, cudaMemcpyDeviceToHost, stream_);
       if (e == cudaSuccess)
         e = cudaEventRecord(arrived, stream_);
-      while (e == cudaSuccess && (e = cudaEventQuery(arrived)) == cudaErrorNotReady) {
-        cudaGetLastError(); // "not ready" is no error
-        std::this_thread::yield();
-        e = cudaSuccess;
-      }
+      if (e == cudaSuccess)
+        e = cudaEventSynchronize(arrived);
       if (e == cudaSuccess)
         std::memcpy(reinterpret_cast<unsigned char *>(host) + at, slot, n);
     }

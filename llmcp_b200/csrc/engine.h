@@ -106,6 +106,9 @@ public:
   // out_tokens_host[steps][batch]; device_ms, if not null, the CUDA-event time of the loop.
   void generate_batch(const int64_t *first_tokens_host, int64_t position, int64_t steps, int64_t *out_tokens_host,
                       float *device_ms);
+  // Takes the pinned slots (16 MB) that the logits of many rows pass through on their way to pageable memory, if a call
+  // of this engine can have so many (forward_all up to its capacity, decode_batch); else the first such call takes them.
+  void prepare_rows_to_host() noexcept;
   void reset_state();
   // Host <-> device copies of the three state buffers in the reference's layouts:
   // kv [full, 2, kv_heads, capacity, head_dim] bf16, delta [linear, v_heads, k_dim, v_dim] f32,
@@ -232,7 +235,7 @@ private:
   int64_t *token_pinned_ = nullptr;
   void rows_to_host(float *host, const float *device, size_t bytes); // complete once the stream is synchronised
   void take_stage() noexcept;
-  unsigned char *stage_pinned_ = nullptr; // rows_to_host: made with a batch engine whose steps need it, else by the first such call
+  unsigned char *stage_pinned_ = nullptr; // pinned slots of rows_to_host
   int64_t *position_dev_ = nullptr; // device scalar: start position of the running call
   // Inputs of the one-token step behind position_dev_ in one device block: token, cos row, sin row.
   int64_t *dec_tokens_ = nullptr;
