@@ -168,7 +168,7 @@ def test_attention_prefill_on_tensor_cores(fast_mode, S, position):
 
 @pytest.mark.parametrize("S,nk,nv", [(64, 16, 32), (1024, 16, 32), (33, 16, 16), (2, 2, 8)])
 def test_gated_delta_net_prefill_fast(fast_mode, S, nk, nv):
-    """Prefill recurrence with the state rows of a column split over four lanes and fused multiply-adds:
+    """Prefill recurrence with the state rows of two columns split over eight lanes and fused multiply-adds:
     against the oracle, outputs within a bf16 step or two, the final state to f32 rounding noise, and
     the golden vectors within the reference's own tolerance."""
     dk = dv = 128
